@@ -396,6 +396,25 @@ void drop_graphs(cwa_sim* s) {
 }
 
 // ---- passes (enqueue only) ----
+// Whether the density and force passes run with four lanes a particle.
+// Small sims leave the GPU idle and each pass lasts as long as its longest
+// thread, so they share a particle among lanes; the team forms issue more
+// instructions in all, so larger sims keep one thread.  Measured step times
+// (us; one sim, and per step with three sims' steps interleaved; one thread /
+// four lanes, dam break, z cells of h):
+//    4,096 particles: 37 / 28 and 13.9 / 11.0
+//    8,000:           47 / 30 and 18.3 / 12.8
+//   18,816:           49 / 36 and 21.1 / 18.4
+//   32,768:           43 / 47 and 28.2 / 25.7
+//   64,000:           60 / 71 and 37.2 / 43.3
+// (Two lanes lie between: 38 and 17.2 at 18,816, but 5% slower than one thread
+// at 32,768 when uploads interleave.)  The work-queue option keeps its own
+// form.
+bool use_team(const cwa_sim* s) {
+  constexpr int32_t kTeamMaxParticles = 24 * 1024;
+  return !s->opt.nb_queue && s->n_total <= kTeamMaxParticles;
+}
+
 NbArgs nb_args(cwa_sim* s) {
   NbArgs a;
   a.pos = s->P[s->cur];
@@ -424,6 +443,7 @@ NbArgs nb_args(cwa_sim* s) {
   a.force_minb = s->opt.nb_force_minb ? s->opt.nb_force_minb : 9;
   a.order = s->d_porder;
   a.queue = s->opt.nb_queue ? s->d_queue : nullptr;
+  a.team = use_team(s);
   return a;
 }
 

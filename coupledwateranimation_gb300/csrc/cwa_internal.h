@@ -163,15 +163,18 @@ cudaError_t launch_point_rank(const int32_t* key, const int32_t* slot, const int
 // density pass and read by force: nine row masks per particle, word
 // r * n_total + i holding particle i's hits in candidate row r as bits
 // (bit b = the candidate at the row's cell-based start + b).  nbr_cnt holds
-// the rows with a nonzero mask (bit r), the only words force reads, or -1
-// when some row's window reaches past bit 63 (force then rescans the
-// particle's rows).
+// the rows with a nonzero mask (bit r), the only words force reads.  Where
+// some row's window would reach past bit 63, the density pass sets
+// kWindowMasks and the particle's bits count from its row windows' starts
+// instead, which force recomputes from the same position; -1 marks a window
+// of more than 64 candidates (force then rescans the particle's rows).
 // The Verlet list (pairs within h (1 + skin) at the last rebuild) holds
 // 16-bit codes (row << 12 | offset from the row's cell-based start), entry k
 // of particle i at list[k * n_total + i]; a count of kMaxVerlet + 1 marks an
 // overflowed list, whose reader rescans the particle's rows.
 constexpr int kNbRows = 9;
 constexpr int kMaskBits = 64;
+constexpr int kWindowMasks = 1 << kNbRows;
 typedef uint64_t RowMask;  // one candidate row's hits, bit b = the candidate at the row's cell-based start + b
 constexpr int kMaxVerlet = 128;
 struct NbArgs {
@@ -205,6 +208,7 @@ struct NbArgs {
   // queue[1] (force), zeroed before each launch, and run tiles[order[t]].
   const int32_t* order;
   int32_t* queue;
+  bool team;            // several lanes a particle (small sims)
 };
 // Candidate scan: the per-step density + row masks, or (list_mode) the
 // Verlet list, run only when *flag is set.

@@ -122,16 +122,22 @@ __device__ __forceinline__ void row_bases(const SceneDev* S, const int32_t* __re
 // radius carries a 2^-10 margin (about h / 1024 of slack in the window), so
 // neither float rounding nor the approximate square root t * rsqrt(t)
 // (relative error ~1e-7) ever drops a pair.
-__device__ __forceinline__ void row_ranges(const SceneDev* S, const int32_t* __restrict__ start, float4 p,
-                                           CellCoord c, float rad2, int b[9], int e[9]) {
-  const int nz = S->dims[2];
-  const float x0f = S->lo[0] + (float)c.x * S->cell;
-  const float y0f = S->lo[1] + (float)c.y * S->cell;
-  const float dxm = fmaxf(p.x - x0f, 0.0f), dxp = fmaxf(x0f + S->cell - p.x, 0.0f);
-  const float dym = fmaxf(p.y - y0f, 0.0f), dyp = fmaxf(y0f + S->cell - p.y, 0.0f);
-  const float zl = p.z - S->lo[2], izc = S->inv_cellz, zmax = (float)(nz - 1);
-#pragma unroll
-  for (int r = 0; r < 9; ++r) {
+struct RowWindows {
+  float dxm, dxp, dym, dyp, zl, izc, zmax, rad2;
+  __device__ __forceinline__ RowWindows(const SceneDev* S, float4 p, CellCoord c, float r2) {
+    const float x0f = S->lo[0] + (float)c.x * S->cell;
+    const float y0f = S->lo[1] + (float)c.y * S->cell;
+    dxm = fmaxf(p.x - x0f, 0.0f);
+    dxp = fmaxf(x0f + S->cell - p.x, 0.0f);
+    dym = fmaxf(p.y - y0f, 0.0f);
+    dyp = fmaxf(y0f + S->cell - p.y, 0.0f);
+    zl = p.z - S->lo[2];
+    izc = S->inv_cellz;
+    zmax = (float)(S->dims[2] - 1);
+    rad2 = r2;
+  }
+  __device__ __forceinline__ void range(const SceneDev* S, const int32_t* __restrict__ start, CellCoord c, int r,
+                                        int& b, int& e) const {
     const int dx = r / 3 - 1, dy = r % 3 - 1;
     const float ddx = dx < 0 ? dxm : (dx > 0 ? dxp : 0.0f);
     const float ddy = dy < 0 ? dym : (dy > 0 ? dyp : 0.0f);
@@ -142,9 +148,16 @@ __device__ __forceinline__ void row_ranges(const SceneDev* S, const int32_t* __r
     const int z0 = (int)fminf(fmaxf(floorf((zl - w) * izc), 0.0f), zmax);
     const int z1 = (int)fminf(fmaxf(floorf((zl + w) * izc), 0.0f), zmax);
     const int row = row_id(S, c, r);
-    b[r] = ok ? __ldg(start + row + z0) : 0;
-    e[r] = ok ? __ldg(start + row + z1 + 1) : 0;
+    b = ok ? __ldg(start + row + z0) : 0;
+    e = ok ? __ldg(start + row + z1 + 1) : 0;
   }
+};
+
+__device__ __forceinline__ void row_ranges(const SceneDev* S, const int32_t* __restrict__ start, float4 p,
+                                           CellCoord c, float rad2, int b[9], int e[9]) {
+  const RowWindows w(S, p, c, rad2);
+#pragma unroll
+  for (int r = 0; r < 9; ++r) w.range(S, start, c, r, b[r], e[r]);
 }
 
 __device__ __forceinline__ float uv_s(const SceneDev* S, float x) { return x * S->uvs[0] + S->uvo[0]; }
@@ -333,7 +346,7 @@ __device__ __forceinline__ T scan_row(Load load, int len, uint32_t code0, T px, 
 // hits and the hits themselves as bits of the row window (bit o = candidate
 // o; candidates 64 and up are tested and summed but get no bit).  The tests
 // only set register bits, so no lane stores anything per candidate.
-template <class T, class Load>
+template <int U, class T, class Load>
 __device__ __forceinline__ T scan_row_bits(Load load, int len, T px, T py, T pz, T hit2, RowMask& bits) {
   T part = (T)0;
   uint32_t lo = 0u, hi = 0u;
@@ -344,7 +357,7 @@ __device__ __forceinline__ T scan_row_bits(Load load, int len, T px, T py, T pz,
     // a deeper unroll spends its time in the remainder loop.  The candidate
     // pass took 168 us unrolled by 4, 154 by 2, 165 by 1, 167 by 3 and 192
     // by 8 at C1.
-#pragma unroll 2
+#pragma unroll U
     for (int o = 0; o < n; ++o) {
       const float4 pj = load(c0 + o);
       const T dx = px - (T)pj.x, dy = py - (T)pj.y, dz = pz - (T)pj.z;
@@ -444,6 +457,19 @@ __device__ __forceinline__ int scan_tile(
   Sum<P> acc;
   bool overflow = false;
   int hits = 0;  // rows with a nonzero mask (bit r)
+  if (MODE == MODE_DENSITY) {
+    // In a dense spot the candidates below a window can push it past its
+    // row's 64 bits; such a particle's masks count from the windows' own
+    // starts (kWindowMasks), which force recomputes.
+    int reach = 0;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) reach = max(reach, e[r] - base[r]);
+    if (reach > kMaskBits) {
+      hits = kWindowMasks;
+#pragma unroll
+      for (int r = 0; r < 9; ++r) base[r] = b[r];
+    }
+  }
 #pragma unroll
   for (int r = 0; r < 9; ++r) {
     int len = e[r] - b[r];
@@ -464,10 +490,10 @@ __device__ __forceinline__ int scan_tile(
       if (len > 0) {
         if (in_stage) {
           const uint32_t a0 = smem_u32(cand);
-          part = scan_row_bits<T>([&](int o) { return lds128(a0 + 16u * (uint32_t)o); }, len, px, py, pz, hit2,
+          part = scan_row_bits<2, T>([&](int o) { return lds128(a0 + 16u * (uint32_t)o); }, len, px, py, pz, hit2,
                                   bits);
         } else
-          part = scan_row_bits<T>([&](int o) { return __ldg(cand + o); }, len, px, py, pz, hit2, bits);
+          part = scan_row_bits<2, T>([&](int o) { return __ldg(cand + o); }, len, px, py, pz, hit2, bits);
       }
       overflow |= off0 + len > kMaskBits;
       const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
@@ -720,14 +746,145 @@ struct Acc3 {
   }
 };
 
+// One particle's pair sums of the force pass: spiky pressure gradient and
+// viscosity Laplacian over neighbours j.
+template <int P>
+struct PairSums {
+  using T = Real<P>;
+  T px, py, pz, vx, vy, vz, pres, h;
+  Acc3<P> fp, fv;
+  __device__ __forceinline__ void init(const SceneDev* S, float4 pi, float4 vi, float p) {
+    px = pi.x;
+    py = pi.y;
+    pz = pi.z;
+    vx = vi.x;
+    vy = vi.y;
+    vz = vi.z;
+    pres = p;
+    h = (T)S->h;
+  }
+  __device__ __forceinline__ void pair(float4 pj, float4 vj, T irho, T pres_j) {
+    const T dx = px - (T)pj.x, dy = py - (T)pj.y, dz = pz - (T)pj.z;
+    const T r2 = dx * dx + dy * dy + dz * dz;
+    const T inv_r = r2 > (T)0 ? inv_sqrt(r2) : (T)0;  // normalize(0) := 0
+    const T r = r2 * inv_r;
+    const T hr = h - r;
+    const T sp = (pres + pres_j) * irho * hr * hr * inv_r;
+    fp.add(sp * dx, sp * dy, sp * dz);
+    const T sv = irho * hr;
+    fv.add(sv * ((T)vj.x - vx), sv * ((T)vj.y - vy), sv * ((T)vj.z - vz));
+  }
+  __device__ __forceinline__ void flush() {
+    fp.flush();
+    fv.flush();
+  }
+};
+
+// The arrays a pair's neighbour data comes from: FP32 modes read the density
+// pass's records, FP64 gathers pos, vel and (rho, p) and divides in double.
+struct PairArrays {
+  const float4* __restrict__ pos;
+  const float4* __restrict__ vel;
+  const float2* __restrict__ rho_p;
+  const float4* __restrict__ xpair;
+  const float4* __restrict__ vpair;
+};
+
+template <int P>
+__device__ __forceinline__ void pair_global(PairSums<P>& s, const PairArrays& a, int j) {
+  using T = Real<P>;
+  if (P == CWA_PREC_FP64) {
+    const float2 rpj = __ldg(a.rho_p + j);
+    s.pair(__ldg(a.pos + j), __ldg(a.vel + j), recip((T)rpj.x), (T)rpj.y);
+  } else {
+    const float4 xj = __ldg(a.xpair + j), vj = __ldg(a.vpair + j);
+    s.pair(xj, vj, (T)vj.w, (T)xj.w);
+  }
+}
+
+// Adds the pairs of the hits in m (bit b = candidate j0 + b), lowest bit
+// first; U hits' gathers are in flight at a time.
+template <int P, int U, class M>
+__device__ __forceinline__ void add_hits(PairSums<P>& s, const PairArrays& a, int j0, M m) {
+#pragma unroll 1
+  while (m) {
+    int js[U];
+    int k = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      js[u] = j0 + (m ? __ffsll((long long)m) - 1 : 0);
+      k += m != 0;
+      m &= m - 1;
+    }
+    if (P == CWA_PREC_FP64) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < k) pair_global<P>(s, a, js[u]);
+    } else {
+      float4 xj[U], vj[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        xj[u] = __ldg(a.xpair + js[u]);
+        vj[u] = __ldg(a.vpair + js[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < k) s.pair(xj[u], vj[u], vj[u].w, xj[u].w);
+    }
+  }
+}
+
+// Candidate row r of a particle in a dense spot (kWindowMasks, or -1: a row
+// window of more than 64 candidates).  With masks, their bits count from the
+// row window's start; without, the window is tested again, 32 candidates at a
+// time with U loads in flight.  The caller folds the sums once a row.
+// Such particles are few but sit on the pass's critical path: testing each
+// candidate and gathering its hit at once, over every z cell a neighbour
+// could occupy, cost one dependent round trip a candidate and kept single
+// warps running 40 us past the others (force 160 -> 127 us in the 1M-particle
+// run while the sheet of surface particles is dense).
+template <int P, int U>
+__device__ __forceinline__ void dense_row(PairSums<P>& s, const PairArrays& a, const SceneDev* S,
+                                          const int32_t* __restrict__ start, const RowWindows& w, CellCoord c, int i,
+                                          int r, int cnt, const RowMask* __restrict__ nbm, int32_t n_total) {
+  using T = Real<P>;
+  int b, e;
+  w.range(S, start, c, r, b, e);
+  if (cnt >= 0) {
+    RowMask m = (cnt >> r) & 1 ? __ldg(nbm + (size_t)r * n_total + i) : (RowMask)0u;
+    if (r == 4) m &= ~((RowMask)1u << (i - b));  // the particle itself
+    add_hits<P, U>(s, a, b, m);
+    return;
+  }
+  const T h2 = s.h * s.h;
+#pragma unroll 1
+  for (; b < e; b += 32) {
+    const int n = min(e - b, 32);
+    uint32_t m = 0u;
+#pragma unroll 1
+    for (int o = 0; o < n; o += U) {
+      float4 pj[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) pj[u] = __ldg(a.pos + b + min(o + u, n - 1));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const T dx = s.px - (T)pj[u].x, dy = s.py - (T)pj[u].y, dz = s.pz - (T)pj[u].z;
+        T q = fma(-dx, dx, h2);
+        q = fma(-dy, dy, q);
+        q = fma(-dz, dz, q);
+        if (q > (T)0 && o + u < n && b + o + u != i) m |= 1u << (o + u);
+      }
+    }
+    add_hits<P, U>(s, a, b, m);
+  }
+}
+
 // force: spiky pressure gradient + viscosity Laplacian over the step's hits
-// (the row masks), then the preset's extra terms.  A particle whose masks
-// overflowed rescans the rows of its cell over every z cell a neighbour can
-// occupy.  Neighbour data comes from global memory (L1-resident for the most
-// part: a CTA's particles share their candidate rows).  Staging the rows'
-// records in shared memory, as the candidate scan does, measured slower
-// here: 48 KB of stage per CTA halves the resident warps this latency-bound
-// loop needs.
+// (the row masks), then the preset's extra terms.  Neighbour data comes from
+// global memory (L1-resident for the most part: a CTA's particles share their
+// candidate rows).  Staging the rows' records in shared memory, as the
+// candidate scan does, measured slower here: 48 KB of stage per CTA halves
+// the resident warps this latency-bound loop needs.
 template <int P>
 __device__ __forceinline__ void force_tile(
     RowMask (&s_w)[kNbRows][kNbThreads], int32_t (&s_jb)[kNbRows][kNbThreads], const Tile tl,
@@ -745,38 +902,14 @@ __device__ __forceinline__ void force_tile(
   const float4 pi = P == CWA_PREC_FP64 ? __ldg(pos + i) : __ldg(xpair + i);
   const float4 vi = P == CWA_PREC_FP64 ? __ldg(vel + i) : __ldg(vpair + i);
   const float2 rpi = __ldg(rho_p + i);
-  const T hh = (T)S->h;
-  const T h2 = hh * hh;
-  const T px = pi.x, py = pi.y, pz = pi.z;
-  const T vx = vi.x, vy = vi.y, vz = vi.z, pres_i = rpi.y;
-  Acc3<P> fp, fv;
-  auto pair = [&](float4 pj, float4 vj, T irho, T pres_j) {
-    const T dx = px - (T)pj.x, dy = py - (T)pj.y, dz = pz - (T)pj.z;
-    const T r2 = dx * dx + dy * dy + dz * dz;
-    const T inv_r = r2 > (T)0 ? inv_sqrt(r2) : (T)0;  // normalize(0) := 0
-    const T r = r2 * inv_r;
-    const T hr = hh - r;
-    const T sp = (pres_i + pres_j) * irho * hr * hr * inv_r;
-    fp.add(sp * dx, sp * dy, sp * dz);
-    const T sv = irho * hr;
-    fv.add(sv * ((T)vj.x - vx), sv * ((T)vj.y - vy), sv * ((T)vj.z - vz));
-  };
-  // FP32 modes read the density pass's records; FP64 gathers pos, vel and
-  // (rho, p) and divides in double.
-  auto pair_global = [&](int j) {
-    if (P == CWA_PREC_FP64) {
-      const float2 rpj = __ldg(rho_p + j);
-      pair(__ldg(pos + j), __ldg(vel + j), recip((T)rpj.x), (T)rpj.y);
-    } else {
-      const float4 xj = __ldg(xpair + j), vj = __ldg(vpair + j);
-      pair(xj, vj, (T)vj.w, (T)xj.w);
-    }
-  };
+  const PairArrays arrays{pos, vel, rho_p, xpair, vpair};
+  PairSums<P> s;
+  s.init(S, pi, vi, rpi.y);
   const int cnt = __ldg(nbr_cnt + i);
   const CellCoord c = cell_of_key(S, __ldg(keys + i));
-  int base[9];
-  row_bases(S, start, c, base);
-  if (cnt >= 0) {
+  if (cnt >= 0 && !(cnt & kWindowMasks)) {
+    int base[9];
+    row_bases(S, start, c, base);
     // The row masks hold the particle itself: row 4 (its own column) at bit
     // i - base[4], cleared here.  Only the nonzero masks are loaded, back to
     // back, and compacted in row order, and
@@ -787,7 +920,7 @@ __device__ __forceinline__ void force_tile(
     for (int r = 0; r < kNbRows; ++r) {
       // cnt: the rows with hits, as bits; the zero rows are not read
       RowMask m = (cnt >> r) & 1 ? __ldg(nbm + (size_t)r * n_total + i) : (RowMask)0u;
-      if (r == 4 && i - base[4] < kMaskBits) m &= ~((RowMask)1u << (i - base[4]));
+      if (r == 4) m &= ~((RowMask)1u << (i - base[4]));
       if (m) {
         s_w[nw][threadIdx.x] = m;
         s_jb[nw][threadIdx.x] = base[r];
@@ -815,34 +948,22 @@ __device__ __forceinline__ void force_tile(
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (js[u] >= 0 && !CWA_DCHECK_FAILED(js[u] < n_total, status)) pair_global(js[u]);
-      fp.flush();
-      fv.flush();
+        if (js[u] >= 0 && !CWA_DCHECK_FAILED(js[u] < n_total, status)) pair_global<P>(s, arrays, js[u]);
+      s.flush();
     }
   } else {
-    const int z1 = min(c.z + S->rz, S->dims[2] - 1);
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-      if (!row_valid(S, c, r)) continue;
-      const int e = __ldg(start + row_id(S, c, r) + z1 + 1);
-      for (int j = base[r]; j < e; ++j) {
-        const float4 pj = __ldg(pos + j);
-        const T dx = px - (T)pj.x, dy = py - (T)pj.y, dz = pz - (T)pj.z;
-        T q = fma(-dx, dx, h2);
-        q = fma(-dy, dy, q);
-        q = fma(-dz, dz, q);
-        if (q > (T)0 && j != i) pair_global(j);
-      }
-      fp.flush();
-      fv.flush();
+    const RowWindows w(S, pi, c, S->hl2);
+#pragma unroll 1
+    for (int r = 0; r < kNbRows; ++r) {
+      dense_row<P, 2>(s, arrays, S, start, w, c, i, r, cnt, nbm, n_total);
+      s.flush();
     }
   }
-  fp.flush();
-  fv.flush();
+  s.flush();
   const T cg = P == CWA_PREC_FP64 ? (T)S->k_grad_d * (T)S->mass : (T)(S->k_grad * S->mass);
   const T cp = (T)0.5 * cg;
-  float fpr[3] = {(float)(cp * fp.x.get()), (float)(cp * fp.y.get()), (float)(cp * fp.z.get())};
-  float fvr[3] = {(float)(cg * fv.x.get()), (float)(cg * fv.y.get()), (float)(cg * fv.z.get())};
+  float fpr[3] = {(float)(cp * s.fp.x.get()), (float)(cp * s.fp.y.get()), (float)(cp * s.fp.z.get())};
+  float fvr[3] = {(float)(cg * s.fv.x.get()), (float)(cg * s.fv.y.get()), (float)(cg * s.fv.z.get())};
   force[i] = force_out(S, i, pi, vi, rpi.x, fpr, fvr, force, wave);
 }
 
@@ -879,6 +1000,262 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
                     nbr_cnt, n_total, xpair, vpair, status);
     }
   }
+}
+
+// ---- team forms: several lanes a particle --------------------------------
+// A scene of a few tens of thousands of particles leaves most of the GPU
+// idle with one thread a particle: every pass lasts as long as its longest
+// thread.  Here T neighbouring lanes share a particle.  The candidate rows
+// are dealt to the lanes (row r to lane r mod T), and so are force's groups of
+// 8 hits; every row's and every group's partial sum is formed by one lane in
+// the order of the one-thread forms, and the partials are folded into the
+// accumulator in the same order on every lane, so the results are the same
+// bits.  No staging: the lanes read candidates through L1, with several loads
+// in flight.  What bounds them is still latency; they trade total issue for a
+// third of the longest thread's chain: the reference scene's step (20,480
+// particles, walls with ~100 particles a cell) went from 88 to 51 us alone
+// and from 34 to 21 us with three sims interleaved, at four lanes.  Launching
+// them as programmatic dependents measured slower (22 against 18.8 us a step
+// at 18,816 particles with three sims interleaved).
+constexpr int kTeamLanes = 4;
+
+template <int T>
+struct Team {
+  static constexpr int kRounds = (kNbRows + T - 1) / T;
+  int lane;        // this thread's place in its team
+  unsigned mask;   // the team's lanes of the warp
+  __device__ __forceinline__ Team() {
+    const int l = threadIdx.x & 31;
+    lane = l & (T - 1);
+    mask = (T == 32 ? 0xffffffffu : ((1u << T) - 1u)) << (l - lane);
+  }
+  template <class V>
+  __device__ __forceinline__ V from(V v, int k) const {
+    return __shfl_sync(mask, v, k, T);
+  }
+  __device__ __forceinline__ int max_all(int v) const {
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) v = max(v, __shfl_xor_sync(mask, v, o, T));
+    return v;
+  }
+  __device__ __forceinline__ int or_all(int v) const {
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) v |= __shfl_xor_sync(mask, v, o, T);
+    return v;
+  }
+  __device__ __forceinline__ int sum_all(int v) const {
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) v += __shfl_xor_sync(mask, v, o, T);
+    return v;
+  }
+};
+
+// The particle of this thread's team, or -1 past the tile's end.  Each tile
+// of blockDim.x particles is shared by T consecutive CTAs.
+template <int T>
+__device__ __forceinline__ int team_particle(const Tile& tl) {
+  const int per = blockDim.x / T;
+  const int i = tl.begin + (blockIdx.x % T) * per + threadIdx.x / T;
+  return i < tl.end ? i : -1;
+}
+
+template <int P, int T>
+__global__ void __launch_bounds__(kNbThreads)
+    k_rho_team(const float4* __restrict__ pos, const int32_t* __restrict__ start, const int32_t* __restrict__ keys,
+               const Tile* __restrict__ tiles, const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
+               float2* __restrict__ rho_p, int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks,
+               int32_t n_total, const float4* __restrict__ vel, float4* __restrict__ xpair,
+               float4* __restrict__ vpair, int32_t* status) {
+  using R = Real<P>;
+  const Tile tl = tiles[blockIdx.x / T];
+  const int i = team_particle<T>(tl);
+  if (i < 0) return;  // whole teams leave together
+  const Team<T> team;
+  const SceneDev* S = scenes + tl.scene;
+  const float4 pi = __ldg(pos + i);
+  const CellCoord c = cell_of_key(S, __ldg(keys + i));
+  const R hh = (R)S->h;
+  const R h2 = hh * hh;
+  const R px = pi.x, py = pi.y, pz = pi.z;
+  const RowWindows w(S, pi, c, S->hl2);
+  const int zb = max(c.z - S->rz, 0);
+  int b[Team<T>::kRounds], e[Team<T>::kRounds], base[Team<T>::kRounds];
+  int reach = 0;
+#pragma unroll
+  for (int q = 0; q < Team<T>::kRounds; ++q) {
+    const int r = q * T + team.lane;
+    b[q] = e[q] = base[q] = 0;
+    if (r < kNbRows) {
+      w.range(S, start, c, r, b[q], e[q]);
+      base[q] = row_valid(S, c, r) ? __ldg(start + row_id(S, c, r) + zb) : 0;
+      reach = max(reach, e[q] - base[q]);
+    }
+  }
+  int hits = team.max_all(reach) > kMaskBits ? kWindowMasks : 0;
+  int overflow = 0;
+  R part[Team<T>::kRounds];
+#pragma unroll
+  for (int q = 0; q < Team<T>::kRounds; ++q) {
+    const int r = q * T + team.lane;
+    part[q] = (R)0;
+    if (r < kNbRows) {
+      const int len = e[q] - b[q];
+      const int off0 = hits & kWindowMasks ? 0 : b[q] - base[q];
+      RowMask bits = 0u;
+      if (len > 0 && !CWA_DCHECK_FAILED(b[q] >= 0 && e[q] <= n_total, status)) {
+        const float4* cand = pos + b[q];
+        part[q] = scan_row_bits<4, R>([&](int o) { return __ldg(cand + o); }, len, px, py, pz, h2, bits);
+      }
+      overflow |= off0 + len > kMaskBits;
+      const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
+      masks[(size_t)r * n_total + i] = m;
+      if (m != 0u) hits |= 1 << r;
+    }
+  }
+  hits = team.or_all(hits);
+  overflow = team.or_all(overflow);
+  Sum<P> acc;
+#pragma unroll
+  for (int r = 0; r < kNbRows; ++r) acc.add(team.from(part[r / T], r % T));
+  if (team.lane != 0) return;
+  list_cnt[i] = overflow ? -1 : hits;
+  const R rho_t = (P == CWA_PREC_FP64 ? (R)S->c_poly6_d : (R)S->c_poly6) * acc.get();
+  const float2 rp = eos(S, (float)rho_t, pi, wave);
+  rho_p[i] = rp;
+  write_pair_rec(xpair, vpair, vel, i, pi, rp);
+}
+
+// Force in the team form, for the cascaded sums only: their partials (8 hits,
+// or a row in a dense spot) split across lanes without changing a rounding;
+// the plain and FP64 sums are one chain over all hits.
+template <int T>
+__global__ void __launch_bounds__(kNbThreads, 6)
+    k_force_team(const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rho_p,
+                 const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
+                 const SceneDev* __restrict__ scenes, const float* __restrict__ wave, float4* __restrict__ force,
+                 const RowMask* __restrict__ nbm, const int32_t* __restrict__ nbr_cnt, int32_t n_total,
+                 const float4* __restrict__ xpair, const float4* __restrict__ vpair, int32_t* status) {
+  constexpr int P = CWA_PREC_COMPENSATED;
+  __shared__ RowMask s_w[kNbRows][kNbThreads / T];
+  __shared__ int32_t s_jb[kNbRows][kNbThreads / T];
+  __shared__ float s_part[kNbThreads][7];  // 7: odd stride, no bank conflicts
+  const Tile tl = tiles[blockIdx.x / T];
+  const int i = team_particle<T>(tl);
+  if (i < 0) return;
+  const Team<T> team;
+  const int tm = threadIdx.x / T;  // the team's column of the shared arrays
+  const SceneDev* S = scenes + tl.scene;
+  const float4 pi = __ldg(xpair + i), vi = __ldg(vpair + i);
+  const float2 rpi = __ldg(rho_p + i);
+  const int cnt = __ldg(nbr_cnt + i);
+  const CellCoord c = cell_of_key(S, __ldg(keys + i));
+  const PairArrays arrays{pos, vel, rho_p, xpair, vpair};
+  PairSums<P> s;
+  s.init(S, pi, vi, rpi.y);
+  // Folds the lanes' partials in lane order: lane c keeps the sums of
+  // components c, c + T, ... of (pressure xyz, viscosity xyz).
+  constexpr int kOwn = (6 + T - 1) / T;
+  Sum<P> own[kOwn];
+  auto fold = [&]() {
+    float* mine = s_part[threadIdx.x];
+    mine[0] = s.fp.px;
+    mine[1] = s.fp.py;
+    mine[2] = s.fp.pz;
+    mine[3] = s.fv.px;
+    mine[4] = s.fv.py;
+    mine[5] = s.fv.pz;
+    s.fp.px = s.fp.py = s.fp.pz = s.fv.px = s.fv.py = s.fv.pz = 0.0f;
+    __syncwarp(team.mask);
+#pragma unroll
+    for (int q = 0; q < kOwn; ++q) {
+      const int comp = min(q * T + team.lane, 5);
+#pragma unroll
+      for (int k = 0; k < T; ++k) own[q].add(s_part[tm * T + k][comp]);
+    }
+    __syncwarp(team.mask);
+  };
+  if (cnt >= 0 && !(cnt & kWindowMasks)) {
+    const int zb = max(c.z - S->rz, 0);
+    int left = 0;
+#pragma unroll
+    for (int q = 0; q < Team<T>::kRounds; ++q) {
+      const int r = q * T + team.lane;
+      if (r < kNbRows) {
+        RowMask m = (cnt >> r) & 1 ? __ldg(nbm + (size_t)r * n_total + i) : (RowMask)0u;
+        const int base = row_valid(S, c, r) ? __ldg(start + row_id(S, c, r) + zb) : 0;
+        if (r == 4) m &= ~((RowMask)1u << (i - base));  // the particle itself
+        s_w[r][tm] = m;
+        s_jb[r][tm] = base;
+        left += __popcll(m);
+      }
+    }
+    left = team.sum_all(left);
+    __syncwarp(team.mask);
+    // lane k sums hits 8k .. 8k + 7 of every 8 T, in order
+    int wi = -1, skip = 8 * team.lane, jb = 0;
+    RowMask cw = 0u;
+    for (int g0 = 0; g0 < left; g0 += 8 * T) {
+      const int n = min(left - g0 - 8 * team.lane, 8);
+      if (n > 0) {
+        // walk to this lane's first hit of the round: whole masks, then bits
+        for (;;) {
+          const int have = __popcll(cw);
+          if (skip < have) break;
+          skip -= have;
+          ++wi;
+          cw = s_w[wi][tm];
+          jb = s_jb[wi][tm];
+        }
+        for (; skip > 0; --skip) cw &= cw - 1u;
+        int js[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          js[u] = i;
+          if (u < n) {
+            while (cw == 0u) {
+              ++wi;
+              cw = s_w[wi][tm];
+              jb = s_jb[wi][tm];
+            }
+            const int j = jb + __ffsll((long long)cw) - 1;
+            cw &= cw - 1u;
+            if (!CWA_DCHECK_FAILED(j >= 0 && j < n_total, status)) js[u] = j;
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+          float4 xj[4], vj[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            xj[u] = __ldg(xpair + js[h + u]);
+            vj[u] = __ldg(vpair + js[h + u]);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (h + u < n) s.pair(xj[u], vj[u], vj[u].w, xj[u].w);
+        }
+        skip = 8 * (T - 1);
+      }
+      fold();
+    }
+  } else {
+    const RowWindows w(S, pi, c, S->hl2);
+#pragma unroll 1
+    for (int q = 0; q < Team<T>::kRounds; ++q) {
+      const int r = q * T + team.lane;
+      if (r < kNbRows) dense_row<P, 4>(s, arrays, S, start, w, c, i, r, cnt, nbm, n_total);
+      fold();
+    }
+  }
+  float sum[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) sum[k] = team.from(own[k / T].get(), k % T);
+  if (team.lane != 0) return;
+  const float cg = S->k_grad * S->mass;
+  const float cp = 0.5f * cg;
+  float fpr[3] = {cp * sum[0], cp * sum[1], cp * sum[2]};
+  float fvr[3] = {cg * sum[3], cg * sum[4], cg * sum[5]};
+  force[i] = force_out(S, i, pi, vi, rpi.x, fpr, fvr, force, wave);
 }
 
 // Grid of a work-queue launch: the CTAs of `kernel` that fit the device at
@@ -923,6 +1300,12 @@ void scan_variant(int minb, const NbArgs& a, uint16_t* list, int32_t* cnt, RowMa
 
 template <int P>
 void dispatch_scan(bool list_mode, const NbArgs& a, cudaStream_t st) {
+  if (!list_mode && a.team) {
+    k_rho_team<P, kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
+        a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.xpair,
+        a.vpair, a.status);
+    return;
+  }
   if (list_mode)
     scan_variant<P, MODE_LIST>(a.scan_minb, a, a.vlist, a.vcnt, nullptr, a.xref, a.flag, nullptr, st);
   else
@@ -946,6 +1329,14 @@ void force_variant(const NbArgs& a, cudaStream_t st) {
 
 template <int P>
 void dispatch_force(const NbArgs& a, cudaStream_t st) {
+  if constexpr (P == CWA_PREC_COMPENSATED) {
+    if (a.team) {
+      k_force_team<kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
+          a.pos, a.vel, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm, a.nbr_cnt, a.n_total,
+          a.xpair, a.vpair, a.status);
+      return;
+    }
+  }
   // FP64 keeps eight CTAs a SM for nine: its 56-register form spills more
   if constexpr (P != CWA_PREC_FP64) {
     if (a.force_minb >= 9) {
