@@ -62,9 +62,11 @@ struct cwa_sim {
   uint16_t* vlist = nullptr;   // kMaxVerlet x n_total codes
   int32_t* vcnt = nullptr;
   float4* XR = nullptr;        // positions at the last rebuild
-  // force's gather records (x, y, z, p), (vx, vy, vz, 1/rho); FP32 modes only
+  // force's gather records (x, y, z, p), (vx, vy, vz, 1/rho); 1/rho is in IR
+  // (double) in FP64 mode
   float4* XP = nullptr;
   float4* VP = nullptr;
+  double* IR = nullptr;
   int32_t* d_flag = nullptr;   // rebuild flag, raised by integrate / uploads
   unsigned long long* d_rebuilds = nullptr;
   void* scan_ws = nullptr;
@@ -435,6 +437,7 @@ NbArgs nb_args(cwa_sim* s) {
   a.xref = s->XR;
   a.xpair = s->XP;
   a.vpair = s->VP;
+  a.irho = s->IR;
   a.n_total = s->n_total;
   a.status = s->d_status;
   a.flag = s->verlet ? s->d_flag : nullptr;
@@ -893,10 +896,9 @@ cwa_status cwa_create(const cwa_sim_options* opt, const cwa_scene_desc* scenes, 
   ALLOC(s->nbm, N * kNbRows);
   ALLOC(s->nbr_cnt, N);
   ALLOC(s->KS, N);
-  if (s->opt.precision != CWA_PREC_FP64) {
-    ALLOC(s->XP, N);
-    ALLOC(s->VP, N);
-  }
+  ALLOC(s->XP, N);
+  ALLOC(s->VP, N);
+  if (s->opt.precision == CWA_PREC_FP64) ALLOC(s->IR, N);
   ALLOC(s->d_flag, 1);
   ALLOC(s->d_rebuilds, 1);
   if (s->verlet) {

@@ -194,9 +194,11 @@ struct NbArgs {
   int32_t* vcnt;
   float4* xref;         // positions at the last rebuild (Verlet mode)
   // (x, y, z, p) and (vx, vy, vz, 1/rho) of every particle, written by the
-  // density pass for force's neighbour gathers (FP32 modes; null in FP64)
+  // density pass for force's neighbour gathers; FP64 has 1/rho in irho
+  // instead (null in the FP32 modes)
   float4* xpair;
   float4* vpair;
+  double* irho;
   int32_t n_total;
   int32_t* status;
   const int32_t* flag;  // rebuild flag (Verlet mode), else null

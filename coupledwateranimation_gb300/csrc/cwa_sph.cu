@@ -81,6 +81,34 @@ __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float recip(float x) { return __fdividef(1.0f, x); }
 __device__ __forceinline__ double recip(double x) { return 1.0 / x; }
 
+// (double)f without the conversion instruction.  GB300 runs every FP64
+// instruction, float <-> double conversions included, at 2 lanes a clock and
+// SM; the integer form runs at 64.  Zeros, denormals, infinities and NaNs
+// take the instruction.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f);
+  if (((u >> 23) + 1u & 0xffu) <= 1u) return (double)f;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u >> 3) & 0x0fffffffu) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ float widen_as(float f, float) { return f; }
+__device__ __forceinline__ double widen_as(float f, double) { return widen(f); }
+
+// a - b in the precision of the third argument's type, the operands being
+// floats.  In double: the float difference is exact unless the operands
+// differ by more than a factor of 2 (positions near a coordinate plane); its
+// error (exact, Knuth's two-sum) is added back there, so the result equals
+// the double difference of the operands, for one integer conversion instead
+// of two conversions and a subtraction in FP64.
+__device__ __forceinline__ float diff_as(float a, float b, float) { return a - b; }
+__device__ __forceinline__ double diff_as(float a, float b, double) {
+  const float d = __fsub_rn(a, b);
+  const float bb = __fsub_rn(d, a);
+  const float e = __fsub_rn(__fsub_rn(a, __fsub_rn(d, bb)), __fadd_rn(b, bb));
+  double x = widen(d);
+  if (fabsf(e) > 0.0f) x += widen(e);
+  return x;
+}
+
 struct CellCoord {
   int x, y, z;
 };
@@ -179,12 +207,16 @@ __device__ __forceinline__ float2 eos(const SceneDev* S, float rho, float4 pi, c
 
 // Force's gather records of particle i: (x, y, z, p) and (vx, vy, vz, 1/rho),
 // so a pair costs two aligned 16-byte gathers; 1/rho uses force's recip.
+// FP64 keeps 1/rho in double beside them: one division a particle instead of
+// one a pair.
+template <int P>
 __device__ __forceinline__ void write_pair_rec(float4* __restrict__ xp, float4* __restrict__ vp,
-                                               const float4* __restrict__ vel, int i, float4 pi, float2 rp) {
-  if (!xp) return;
+                                               double* __restrict__ irho, const float4* __restrict__ vel, int i,
+                                               float4 pi, float2 rp) {
   const float4 v = __ldg(vel + i);
   xp[i] = make_float4(pi.x, pi.y, pi.z, rp.y);
-  vp[i] = make_float4(v.x, v.y, v.z, recip(rp.x));
+  vp[i] = make_float4(v.x, v.y, v.z, P == CWA_PREC_FP64 ? 0.0f : recip(rp.x));
+  if (P == CWA_PREC_FP64) irho[i] = recip((double)rp.x);
 }
 
 // ---- shared-memory staging with bulk TMA copies --------------------------
@@ -379,6 +411,64 @@ __device__ __forceinline__ T scan_row_bits(Load load, int len, T px, T py, T pz,
   return part;
 }
 
+// The same row in FP64.  A float test against the margin radius (which no
+// hit of the double test fails: the margin is 2^-10, the float distance's
+// error 2^-22) picks the candidates, and only those run in double, in order;
+// the sum and the bits are those of testing every candidate in double.
+// FP64 instructions (2 lanes a clock and SM) bound this pass: ~5 for each of
+// ~37 candidates a particle instead of ~12 for each of ~130.  With force's
+// conversions and division taken out of its pair loop (widen, diff_as, the
+// stored 1/rho: ~26 FP64 instructions a pair instead of ~43), the grid,
+// density and force of 68,265 particles went from 432 to 209 us.
+template <int U, class Load>
+__device__ __forceinline__ double scan_row_fp64(Load load, int len, float4 pi, double hit2, float rad2,
+                                                RowMask& bits) {
+  double part = 0.0;
+  uint32_t lo = 0u, hi = 0u;
+  for (int c0 = 0; c0 < len; c0 += 32) {
+    const int n = min(len - c0, 32);
+    uint32_t near = 0u, m = 0u, bit = 1u;
+#pragma unroll U
+    for (int o = 0; o < n; ++o) {
+      const float4 pj = load(c0 + o);
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      if (dx * dx + dy * dy + dz * dz < rad2) near |= bit;
+      bit <<= 1;
+    }
+    while (near) {
+      const int o = __ffs((int)near) - 1;
+      near &= near - 1u;
+      const float4 pj = load(c0 + o);
+      const double dx = diff_as(pi.x, pj.x, 0.0), dy = diff_as(pi.y, pj.y, 0.0), dz = diff_as(pi.z, pj.z, 0.0);
+      double q = fma(-dx, dx, hit2);
+      q = fma(-dy, dy, q);
+      q = fma(-dz, dz, q);
+      const int top = __double2hiint(q);  // q > 0, tested on its bits
+      if (top >= 0 && (top | __double2loint(q)) != 0 && top < 0x7ff00000) {
+        part = fma(q * q, q, part);
+        m |= 1u << o;
+      }
+    }
+    if (c0 == 0)
+      lo = m;
+    else if (c0 == 32)
+      hi = m;
+  }
+  bits = ((RowMask)hi << 32) | lo;
+  return part;
+}
+
+// One candidate row in the precision P (hit2 = h^2, rad2 >= its float
+// rounding with a margin).
+template <int P, int U, class Load>
+__device__ __forceinline__ Real<P> scan_row_prec(Load load, int len, float4 pi, Real<P> hit2, float rad2,
+                                                 RowMask& bits) {
+  if constexpr (P == CWA_PREC_FP64)
+    return scan_row_fp64<U>(load, len, pi, hit2, rad2, bits);
+  else
+    return scan_row_bits<U, float>(load, len, pi.x, pi.y, pi.z, hit2, bits);
+}
+
 // Candidate scan.  MODE_DENSITY (per-step mode): radius h, density + this
 // step's row masks.  MODE_LIST (Verlet mode, only when the rebuild flag is
 // up): radius h (1 + skin), the Verlet list and the rebuild positions.
@@ -409,7 +499,7 @@ __device__ __forceinline__ int scan_tile(
     const float* __restrict__ wave, float2* __restrict__ rho_p, uint16_t* __restrict__ list,
     int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total,
     int32_t* status, int32_t allow_stage, const float4* __restrict__ vel, float4* __restrict__ xpair,
-    float4* __restrict__ vpair) {
+    float4* __restrict__ vpair, double* __restrict__ irho) {
   using T = Real<P>;
   constexpr int kCap = kMaxVerlet;  // the Verlet list build's codes per particle
   // The list build (rare: Verlet rebuilds only) reads candidates from global
@@ -490,10 +580,10 @@ __device__ __forceinline__ int scan_tile(
       if (len > 0) {
         if (in_stage) {
           const uint32_t a0 = smem_u32(cand);
-          part = scan_row_bits<2, T>([&](int o) { return lds128(a0 + 16u * (uint32_t)o); }, len, px, py, pz, hit2,
-                                  bits);
+          part = scan_row_prec<P, 2>([&](int o) { return lds128(a0 + 16u * (uint32_t)o); }, len, pi, hit2, S->hs2,
+                                     bits);
         } else
-          part = scan_row_bits<2, T>([&](int o) { return __ldg(cand + o); }, len, px, py, pz, hit2, bits);
+          part = scan_row_prec<P, 2>([&](int o) { return __ldg(cand + o); }, len, pi, hit2, S->hs2, bits);
       }
       overflow |= off0 + len > kMaskBits;
       const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
@@ -530,7 +620,7 @@ __device__ __forceinline__ int scan_tile(
     const T rho_t = (P == CWA_PREC_FP64 ? (T)S->c_poly6_d : (T)S->c_poly6) * acc.get();
     const float2 rp = eos(S, (float)rho_t, pi, wave);
     rho_p[i] = rp;
-    write_pair_rec(xpair, vpair, vel, i, pi, rp);
+    write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
   }
   return used;
 }
@@ -548,14 +638,15 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
                  RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total, int32_t* status,
                  const int32_t* __restrict__ flag,
                  int32_t allow_stage, const float4* __restrict__ vel, float4* __restrict__ xpair,
-                 float4* __restrict__ vpair, const int32_t* __restrict__ order, int32_t* queue, int32_t n_tiles) {
+                 float4* __restrict__ vpair, double* __restrict__ irho, const int32_t* __restrict__ order, int32_t* queue,
+                 int32_t n_tiles) {
   __shared__ ScanShared<MODE> sh;
   __shared__ int32_t s_next;
   if (MODE == MODE_LIST && flag && __ldg(flag) == 0) return;  // no rebuild this step
   if (threadIdx.x == 0) mbar_init(&sh.bar, 1);
   if constexpr (!WQ || MODE != MODE_DENSITY) {
     scan_tile<P, MODE>(sh, tiles[blockIdx.x], 0u, pos, start, keys, scenes, wave, rho_p, list, list_cnt, masks,
-                       xref, n_total, status, allow_stage, vel, xpair, vpair);
+                       xref, n_total, status, allow_stage, vel, xpair, vpair, irho);
     return;
   }
   uint32_t parity = 0u;
@@ -567,7 +658,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
     if (t >= n_tiles) break;
     const int used = scan_tile<P, MODE>(sh, tiles[__ldg(order + t)], parity, pos, start, keys, scenes, wave, rho_p,
                                         list, list_cnt, masks, xref, n_total, status, allow_stage, vel, xpair,
-                                        vpair);
+                                        vpair, irho);
     if (__syncthreads_or(used & 2)) break;  // a staging wait timed out (status set): stop taking tiles
     if (used & 1) parity ^= 1u;
   }
@@ -586,7 +677,7 @@ __global__ void __launch_bounds__(kNbThreads, 8)
                float2* __restrict__ rho_p, const uint16_t* __restrict__ vlist,
                const int32_t* __restrict__ vcnt, RowMask* __restrict__ nbm, int32_t* __restrict__ nbr_cnt,
                int32_t n_total, const float4* __restrict__ vel, float4* __restrict__ xpair,
-               float4* __restrict__ vpair) {
+               float4* __restrict__ vpair, double* __restrict__ irho) {
   using T = Real<P>;
   __shared__ int32_t s_rb[9][kNbThreads];
   __shared__ RowMask s_m[kNbRows][kNbThreads];  // this step's row masks
@@ -668,7 +759,7 @@ __global__ void __launch_bounds__(kNbThreads, 8)
   const T rho_t = (P == CWA_PREC_FP64 ? (T)S->c_poly6_d : (T)S->c_poly6) * acc.get();
   const float2 rp = eos(S, (float)rho_t, pi, wave);
   rho_p[i] = rp;
-  write_pair_rec(xpair, vpair, vel, i, pi, rp);
+  write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
 }
 
 // The force a particle stores: pressure + viscosity sums (already scaled,
@@ -751,7 +842,8 @@ struct Acc3 {
 template <int P>
 struct PairSums {
   using T = Real<P>;
-  T px, py, pz, vx, vy, vz, pres, h;
+  float px, py, pz;
+  T vx, vy, vz, pres, h;
   Acc3<P> fp, fv;
   __device__ __forceinline__ void init(const SceneDev* S, float4 pi, float4 vi, float p) {
     px = pi.x;
@@ -763,16 +855,18 @@ struct PairSums {
     pres = p;
     h = (T)S->h;
   }
-  __device__ __forceinline__ void pair(float4 pj, float4 vj, T irho, T pres_j) {
-    const T dx = px - (T)pj.x, dy = py - (T)pj.y, dz = pz - (T)pj.z;
+  // xj, vj: the neighbour's gather records
+  __device__ __forceinline__ void pair(float4 xj, float4 vj, T irho) {
+    const T z = (T)0;
+    const T dx = diff_as(px, xj.x, z), dy = diff_as(py, xj.y, z), dz = diff_as(pz, xj.z, z);
     const T r2 = dx * dx + dy * dy + dz * dz;
     const T inv_r = r2 > (T)0 ? inv_sqrt(r2) : (T)0;  // normalize(0) := 0
     const T r = r2 * inv_r;
     const T hr = h - r;
-    const T sp = (pres + pres_j) * irho * hr * hr * inv_r;
+    const T sp = (pres + widen_as(xj.w, z)) * irho * hr * hr * inv_r;
     fp.add(sp * dx, sp * dy, sp * dz);
     const T sv = irho * hr;
-    fv.add(sv * ((T)vj.x - vx), sv * ((T)vj.y - vy), sv * ((T)vj.z - vz));
+    fv.add(sv * (widen_as(vj.x, z) - vx), sv * (widen_as(vj.y, z) - vy), sv * (widen_as(vj.z, z) - vz));
   }
   __device__ __forceinline__ void flush() {
     fp.flush();
@@ -780,26 +874,22 @@ struct PairSums {
   }
 };
 
-// The arrays a pair's neighbour data comes from: FP32 modes read the density
-// pass's records, FP64 gathers pos, vel and (rho, p) and divides in double.
+// The arrays a pair's neighbour data comes from (the density pass's records)
+// and the positions.
 struct PairArrays {
   const float4* __restrict__ pos;
-  const float4* __restrict__ vel;
-  const float2* __restrict__ rho_p;
   const float4* __restrict__ xpair;
   const float4* __restrict__ vpair;
+  const double* __restrict__ irho;
 };
 
+// 1/rho of neighbour j in the precision P.
 template <int P>
-__device__ __forceinline__ void pair_global(PairSums<P>& s, const PairArrays& a, int j) {
-  using T = Real<P>;
-  if (P == CWA_PREC_FP64) {
-    const float2 rpj = __ldg(a.rho_p + j);
-    s.pair(__ldg(a.pos + j), __ldg(a.vel + j), recip((T)rpj.x), (T)rpj.y);
-  } else {
-    const float4 xj = __ldg(a.xpair + j), vj = __ldg(a.vpair + j);
-    s.pair(xj, vj, (T)vj.w, (T)xj.w);
-  }
+__device__ __forceinline__ Real<P> inv_rho(const PairArrays& a, float4 vj, int j) {
+  if constexpr (P == CWA_PREC_FP64)
+    return __ldg(a.irho + j);
+  else
+    return vj.w;
 }
 
 // Adds the pairs of the hits in m (bit b = candidate j0 + b), lowest bit
@@ -816,21 +906,17 @@ __device__ __forceinline__ void add_hits(PairSums<P>& s, const PairArrays& a, in
       k += m != 0;
       m &= m - 1;
     }
-    if (P == CWA_PREC_FP64) {
+    float4 xj[U], vj[U];
+    Real<P> ir[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (u < k) pair_global<P>(s, a, js[u]);
-    } else {
-      float4 xj[U], vj[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        xj[u] = __ldg(a.xpair + js[u]);
-        vj[u] = __ldg(a.vpair + js[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (u < k) s.pair(xj[u], vj[u], vj[u].w, xj[u].w);
+    for (int u = 0; u < U; ++u) {
+      xj[u] = __ldg(a.xpair + js[u]);
+      vj[u] = __ldg(a.vpair + js[u]);
+      ir[u] = inv_rho<P>(a, vj[u], js[u]);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < k) s.pair(xj[u], vj[u], ir[u]);
   }
 }
 
@@ -868,7 +954,7 @@ __device__ __forceinline__ void dense_row(PairSums<P>& s, const PairArrays& a, c
       for (int u = 0; u < U; ++u) pj[u] = __ldg(a.pos + b + min(o + u, n - 1));
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const T dx = s.px - (T)pj[u].x, dy = s.py - (T)pj[u].y, dz = s.pz - (T)pj[u].z;
+        const T dx = diff_as(s.px, pj[u].x, h2), dy = diff_as(s.py, pj[u].y, h2), dz = diff_as(s.pz, pj[u].z, h2);
         T q = fma(-dx, dx, h2);
         q = fma(-dy, dy, q);
         q = fma(-dz, dz, q);
@@ -888,21 +974,20 @@ __device__ __forceinline__ void dense_row(PairSums<P>& s, const PairArrays& a, c
 template <int P>
 __device__ __forceinline__ void force_tile(
     RowMask (&s_w)[kNbRows][kNbThreads], int32_t (&s_jb)[kNbRows][kNbThreads], const Tile tl,
-    const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rho_p,
+    const float4* __restrict__ pos, const float2* __restrict__ rho_p,
     const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const SceneDev* __restrict__ scenes,
     const float* __restrict__ wave, float4* __restrict__ force, const RowMask* __restrict__ nbm,
     const int32_t* __restrict__ nbr_cnt, int32_t n_total, const float4* __restrict__ xpair,
-    const float4* __restrict__ vpair, int32_t* status) {
+    const float4* __restrict__ vpair, const double* __restrict__ irho, int32_t* status) {
   using T = Real<P>;
   const SceneDev* S = scenes + tl.scene;
   const int i = tl.begin + threadIdx.x;
   if (i >= tl.end) return;
-  // FP32 modes read the particle's own position and velocity from its gather
-  // records (the same floats, and lines its neighbours' gathers share)
-  const float4 pi = P == CWA_PREC_FP64 ? __ldg(pos + i) : __ldg(xpair + i);
-  const float4 vi = P == CWA_PREC_FP64 ? __ldg(vel + i) : __ldg(vpair + i);
+  // the particle's own position and velocity come from its gather records
+  // (the same floats, and lines its neighbours' gathers share)
+  const float4 pi = __ldg(xpair + i), vi = __ldg(vpair + i);
   const float2 rpi = __ldg(rho_p + i);
-  const PairArrays arrays{pos, vel, rho_p, xpair, vpair};
+  const PairArrays arrays{pos, xpair, vpair, irho};
   PairSums<P> s;
   s.init(S, pi, vi, rpi.y);
   const int cnt = __ldg(nbr_cnt + i);
@@ -948,7 +1033,10 @@ __device__ __forceinline__ void force_tile(
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (js[u] >= 0 && !CWA_DCHECK_FAILED(js[u] < n_total, status)) pair_global<P>(s, arrays, js[u]);
+        if (js[u] >= 0 && !CWA_DCHECK_FAILED(js[u] < n_total, status)) {
+          const float4 xj = __ldg(xpair + js[u]), vj = __ldg(vpair + js[u]);
+          s.pair(xj, vj, inv_rho<P>(arrays, vj, js[u]));
+        }
       s.flush();
     }
   } else {
@@ -971,13 +1059,12 @@ __device__ __forceinline__ void force_tile(
 // work-queue form.
 template <int P, int MINB, bool WQ>
 __global__ void __launch_bounds__(kNbThreads, MINB)
-    k_force(const float4* __restrict__ pos, const float4* __restrict__ vel,
-            const float2* __restrict__ rho_p, const int32_t* __restrict__ start,
+    k_force(const float4* __restrict__ pos, const float2* __restrict__ rho_p, const int32_t* __restrict__ start,
             const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
             const SceneDev* __restrict__ scenes, const float* __restrict__ wave, float4* __restrict__ force,
             const RowMask* __restrict__ nbm, const int32_t* __restrict__ nbr_cnt, int32_t n_total,
-            const float4* __restrict__ xpair, const float4* __restrict__ vpair, int32_t* status,
-            const int32_t* __restrict__ order, int32_t* queue, int32_t n_tiles) {
+            const float4* __restrict__ xpair, const float4* __restrict__ vpair, const double* __restrict__ irho,
+            int32_t* status, const int32_t* __restrict__ order, int32_t* queue, int32_t n_tiles) {
   // the particle's nonzero row masks and the index of each mask's bit 0
   // (13.8 KB a CTA; 32-bit masks, 9.2 KB a CTA, measured slower: 209 against
   // 143 us over the C1 run).  The default variant runs nine CTAs a SM at 56
@@ -986,8 +1073,8 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
   __shared__ RowMask s_w[kNbRows][kNbThreads];
   __shared__ int32_t s_jb[kNbRows][kNbThreads];
   if constexpr (!WQ) {
-    force_tile<P>(s_w, s_jb, tiles[blockIdx.x], pos, vel, rho_p, start, keys, scenes, wave, force, nbm, nbr_cnt,
-                  n_total, xpair, vpair, status);
+    force_tile<P>(s_w, s_jb, tiles[blockIdx.x], pos, rho_p, start, keys, scenes, wave, force, nbm, nbr_cnt,
+                  n_total, xpair, vpair, irho, status);
   } else {
     // work-queue form: resident CTAs take tile numbers from *queue
     __shared__ int32_t s_next[2];
@@ -996,8 +1083,8 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
       __syncthreads();  // (two slots: thread 0 refills one while the other is still being read)
       const int t = s_next[it & 1];
       if (t >= n_tiles) break;
-      force_tile<P>(s_w, s_jb, tiles[__ldg(order + t)], pos, vel, rho_p, start, keys, scenes, wave, force, nbm,
-                    nbr_cnt, n_total, xpair, vpair, status);
+      force_tile<P>(s_w, s_jb, tiles[__ldg(order + t)], pos, rho_p, start, keys, scenes, wave, force, nbm,
+                    nbr_cnt, n_total, xpair, vpair, irho, status);
     }
   }
 }
@@ -1065,7 +1152,7 @@ __global__ void __launch_bounds__(kNbThreads)
                const Tile* __restrict__ tiles, const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                float2* __restrict__ rho_p, int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks,
                int32_t n_total, const float4* __restrict__ vel, float4* __restrict__ xpair,
-               float4* __restrict__ vpair, int32_t* status) {
+               float4* __restrict__ vpair, double* __restrict__ irho, int32_t* status) {
   using R = Real<P>;
   const Tile tl = tiles[blockIdx.x / T];
   const int i = team_particle<T>(tl);
@@ -1076,7 +1163,6 @@ __global__ void __launch_bounds__(kNbThreads)
   const CellCoord c = cell_of_key(S, __ldg(keys + i));
   const R hh = (R)S->h;
   const R h2 = hh * hh;
-  const R px = pi.x, py = pi.y, pz = pi.z;
   const RowWindows w(S, pi, c, S->hl2);
   const int zb = max(c.z - S->rz, 0);
   int b[Team<T>::kRounds], e[Team<T>::kRounds], base[Team<T>::kRounds];
@@ -1104,7 +1190,7 @@ __global__ void __launch_bounds__(kNbThreads)
       RowMask bits = 0u;
       if (len > 0 && !CWA_DCHECK_FAILED(b[q] >= 0 && e[q] <= n_total, status)) {
         const float4* cand = pos + b[q];
-        part[q] = scan_row_bits<4, R>([&](int o) { return __ldg(cand + o); }, len, px, py, pz, h2, bits);
+        part[q] = scan_row_prec<P, 4>([&](int o) { return __ldg(cand + o); }, len, pi, h2, S->hs2, bits);
       }
       overflow |= off0 + len > kMaskBits;
       const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
@@ -1122,7 +1208,7 @@ __global__ void __launch_bounds__(kNbThreads)
   const R rho_t = (P == CWA_PREC_FP64 ? (R)S->c_poly6_d : (R)S->c_poly6) * acc.get();
   const float2 rp = eos(S, (float)rho_t, pi, wave);
   rho_p[i] = rp;
-  write_pair_rec(xpair, vpair, vel, i, pi, rp);
+  write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
 }
 
 // Force in the team form, for the cascaded sums only: their partials (8 hits,
@@ -1130,8 +1216,8 @@ __global__ void __launch_bounds__(kNbThreads)
 // the plain and FP64 sums are one chain over all hits.
 template <int T>
 __global__ void __launch_bounds__(kNbThreads, 6)
-    k_force_team(const float4* __restrict__ pos, const float4* __restrict__ vel, const float2* __restrict__ rho_p,
-                 const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
+    k_force_team(const float4* __restrict__ pos, const float2* __restrict__ rho_p, const int32_t* __restrict__ start,
+                 const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
                  const SceneDev* __restrict__ scenes, const float* __restrict__ wave, float4* __restrict__ force,
                  const RowMask* __restrict__ nbm, const int32_t* __restrict__ nbr_cnt, int32_t n_total,
                  const float4* __restrict__ xpair, const float4* __restrict__ vpair, int32_t* status) {
@@ -1149,7 +1235,7 @@ __global__ void __launch_bounds__(kNbThreads, 6)
   const float2 rpi = __ldg(rho_p + i);
   const int cnt = __ldg(nbr_cnt + i);
   const CellCoord c = cell_of_key(S, __ldg(keys + i));
-  const PairArrays arrays{pos, vel, rho_p, xpair, vpair};
+  const PairArrays arrays{pos, xpair, vpair, nullptr};
   PairSums<P> s;
   s.init(S, pi, vi, rpi.y);
   // Folds the lanes' partials in lane order: lane c keeps the sums of
@@ -1232,7 +1318,7 @@ __global__ void __launch_bounds__(kNbThreads, 6)
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            if (h + u < n) s.pair(xj[u], vj[u], vj[u].w, xj[u].w);
+            if (h + u < n) s.pair(xj[u], vj[u], vj[u].w);
         }
         skip = 8 * (T - 1);
       }
@@ -1283,7 +1369,7 @@ void scan_launch_one(const NbArgs& a, uint16_t* list, int32_t* cnt, RowMask* mas
     grid = queue_grid(kern, a.tile_size, a.n_tiles);
   }
   kern<<<grid, a.tile_size, 0, st>>>(a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, list, cnt, masks,
-                                     xref, a.n_total, a.status, flag, a.stage, a.vel, a.xpair, a.vpair, a.order,
+                                     xref, a.n_total, a.status, flag, a.stage, a.vel, a.xpair, a.vpair, a.irho, a.order,
                                      queue, a.n_tiles);
 }
 
@@ -1303,7 +1389,7 @@ void dispatch_scan(bool list_mode, const NbArgs& a, cudaStream_t st) {
   if (!list_mode && a.team) {
     k_rho_team<P, kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
         a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.xpair,
-        a.vpair, a.status);
+        a.vpair, a.irho, a.status);
     return;
   }
   if (list_mode)
@@ -1322,8 +1408,8 @@ void force_variant(const NbArgs& a, cudaStream_t st) {
     cudaMemsetAsync(queue, 0, sizeof(int32_t), st);
     grid = queue_grid(kern, a.tile_size, a.n_tiles);
   }
-  kern<<<grid, a.tile_size, 0, st>>>(a.pos, a.vel, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force,
-                                     a.nbm, a.nbr_cnt, a.n_total, a.xpair, a.vpair, a.status, a.order, queue,
+  kern<<<grid, a.tile_size, 0, st>>>(a.pos, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm,
+                                     a.nbr_cnt, a.n_total, a.xpair, a.vpair, a.irho, a.status, a.order, queue,
                                      a.n_tiles);
 }
 
@@ -1332,7 +1418,7 @@ void dispatch_force(const NbArgs& a, cudaStream_t st) {
   if constexpr (P == CWA_PREC_COMPENSATED) {
     if (a.team) {
       k_force_team<kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
-          a.pos, a.vel, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm, a.nbr_cnt, a.n_total,
+          a.pos, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm, a.nbr_cnt, a.n_total,
           a.xpair, a.vpair, a.status);
       return;
     }
@@ -1367,7 +1453,7 @@ cudaError_t launch_rho_list(int precision, const NbArgs& a, cudaStream_t stream)
 #define CWA_RHO_LIST(P)                                                                                     \
   k_rho_list<P><<<a.n_tiles, a.tile_size, 0, stream>>>(a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave,  \
                                                        a.rho_p, a.vlist, a.vcnt, a.nbm, a.nbr_cnt, a.n_total, \
-                                                       a.vel, a.xpair, a.vpair)
+                                                       a.vel, a.xpair, a.vpair, a.irho)
   switch (precision) {
     case CWA_PREC_FP32: CWA_RHO_LIST(CWA_PREC_FP32); break;
     case CWA_PREC_FP64: CWA_RHO_LIST(CWA_PREC_FP64); break;
