@@ -492,12 +492,14 @@ cudaError_t scan_launch_two_pass(int32_t* in, int32_t* out, int32_t n_in, int32_
   int32_t* sums = reinterpret_cast<int32_t*>(ws.state);  // n_tiles ints in the tile-state area
   const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const dim3 grid(ws.n_tiles), block(kScanBlock);
-  cudaError_t e;
-  if (vec)
-    e = launch_chained(k_tile_sum<true>, grid, block, 0, stream, in, n_in, sums, flag);
-  else
-    e = launch_chained(k_tile_sum<false>, grid, block, 0, stream, in, n_in, sums, flag);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
+  if (ws.n_tiles > 1) {  // a single tile has no totals before it
+    if (vec)
+      e = launch_chained(k_tile_sum<true>, grid, block, 0, stream, in, n_in, sums, flag);
+    else
+      e = launch_chained(k_tile_sum<false>, grid, block, 0, stream, in, n_in, sums, flag);
+    if (e != cudaSuccess) return e;
+  }
   if (zero_input) {
     if (vec)
       e = launch_chained(k_tile_scan<true, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
@@ -509,7 +511,7 @@ cudaError_t scan_launch_two_pass(int32_t* in, int32_t* out, int32_t n_in, int32_
     else
       e = launch_chained(k_tile_scan<false, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
   }
-  if (launches) *launches += 2;
+  if (launches) *launches += ws.n_tiles > 1 ? 2 : 1;
   return e;
 }
 

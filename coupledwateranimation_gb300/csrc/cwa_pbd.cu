@@ -12,10 +12,10 @@
 // The shader accumulates every contact into both boxes with float atomics,
 // so its sums (and the wall terms, added without atomics beside them) depend
 // on thread order.  Here the accumulation is a gather: the query writes each
-// contact once into the lower box's pair slots, a stable counting sort
-// indexes the pairs by their higher box, and PostAnimate sums, per box, its
-// wall terms, then the pairs it owns in slot order, then the pairs it is the
-// partner of in slot order.  Every float operation is rounded to nearest in
+// contact once into the lower box's pair slots and its slot number into a
+// list of the higher box, and PostAnimate sums, per box, its wall terms, then
+// the pairs it owns in slot order, then the pairs it is the partner of in slot
+// order (it sorts its list).  Every float operation is rounded to nearest in
 // a fixed order (round-to-nearest intrinsics), so a step is deterministic
 // and the float32 CPU restatement reproduces it bit for bit.  Cell ids are
 // (i ny + j) nz + k; the shader's (i ny + j) nx + k is the same on its cubic
@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <string>
+#include <vector>
 
 #include "cwa_device.cuh"
 #include "cwa_internal.h"
@@ -63,11 +64,17 @@ __device__ __forceinline__ int cell_c(const PbdConst& c, float p, int a) {
 __device__ __forceinline__ int cell_id(const PbdConst& c, int i, int j, int k) { return (i * c.ny + j) * c.nz + k; }
 
 // COMPUTE_COUNTS / INSERT_BOXES: item q = box * maxc + t is the box's t-th
-// overlapped cell (x-major, z fastest); unused slots get key -1.
+// overlapped cell (x-major, z fastest); unused slots get key -1.  One thread
+// an item, so a box's cell counters are bumped side by side instead of one
+// returned atomic after another.  The box's first thread also clears its
+// contact state and runs PreAnimate (:354-370), which touches nothing the
+// cells come from.
 __global__ void k_pbd_cells(PbdConst c, cwa_pbd_box* __restrict__ boxes, int32_t* __restrict__ ikey,
-                            int32_t* __restrict__ islot, int32_t* __restrict__ count, int32_t* status) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= c.n) return;
+                            int32_t* __restrict__ islot, int32_t* __restrict__ count, int32_t* __restrict__ rcount,
+                            int32_t* status) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= c.n * c.maxc) return;
+  const int b = q / c.maxc, t = q - b * c.maxc;
   cwa_pbd_box& o = boxes[b];
   int lo[3], hi[3];
 #pragma unroll
@@ -75,47 +82,17 @@ __global__ void k_pbd_cells(PbdConst c, cwa_pbd_box* __restrict__ boxes, int32_t
     lo[a] = cell_c(c, fs(o.x[a], o.hw[a]), a);
     hi[a] = cell_c(c, fa(o.x[a], o.hw[a]), a);
   }
-  int t = 0;
-  for (int i = lo[0]; i <= hi[0]; ++i)
-    for (int j = lo[1]; j <= hi[1]; ++j)
-      for (int k = lo[2]; k <= hi[2]; ++k) {
-        if (t < c.maxc) {
-          const int key = cell_id(c, i, j, k);
-          ikey[(size_t)b * c.maxc + t] = key;
-          islot[(size_t)b * c.maxc + t] = count_slot(count, key);
-        } else {
-          atomicOr(status, kStatusBigCell);
-        }
-        ++t;
-      }
-  for (; t < c.maxc; ++t) ikey[(size_t)b * c.maxc + t] = -1;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) o.color[a] = 1.0f;  // InsertBox resets the colour
-}
-
-// Arrival-order insert, then the stable rank (members with a smaller index).
-__global__ void k_pbd_insert(const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
-                             const int32_t* __restrict__ start, int32_t* __restrict__ list, int32_t n_items) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n_items || key[q] < 0) return;
-  list[start[key[q]] + slot[q]] = q;
-}
-
-__global__ void k_pbd_rank(const int32_t* __restrict__ key, const int32_t* __restrict__ start,
-                           const int32_t* __restrict__ list, int32_t* __restrict__ sorted, int32_t n_items) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n_items || key[q] < 0) return;
-  const int b = start[key[q]], e = start[key[q] + 1];
-  int rank = 0;
-  for (int m = b; m < e; ++m) rank += list[m] < q;
-  sorted[b + rank] = q;
-}
-
-// PreAnimate (:354-370).
-__global__ void k_pbd_pre(PbdConst c, cwa_pbd_box* __restrict__ boxes) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= c.n) return;
-  cwa_pbd_box& o = boxes[b];
+  const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1, cells = (hi[0] - lo[0] + 1) * ny * nz;
+  int key = -1;
+  if (t < cells) {
+    const int xy = t / nz;
+    key = cell_id(c, lo[0] + xy / ny, lo[1] + xy % ny, lo[2] + t - xy * nz);
+    islot[q] = count_slot(count, key);
+  }
+  ikey[q] = key;
+  if (t != 0) return;
+  if (cells > c.maxc) atomicOr(status, kStatusBigCell);
+  rcount[b] = 0;
   float v[4];
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
@@ -124,12 +101,33 @@ __global__ void k_pbd_pre(PbdConst c, cwa_pbd_box* __restrict__ boxes) {
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
+    o.color[a] = 1.0f;  // InsertBox resets the colour
     o.dp_n[a] = 0.0f;
     o.dp_t[a] = 0.0f;
     o.p[a] = fa(o.x[a], fm(c.dt, v[a]));
     o.v[a] = v[a];
   }
   o.n = 0.0f;
+}
+
+// Arrival-order insert, then the stable rank (members with a smaller index);
+// the sorted list holds the members' boxes.
+__global__ void k_pbd_insert(const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
+                             const int32_t* __restrict__ start, int32_t* __restrict__ list, int32_t n_items) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n_items || key[q] < 0) return;
+  list[start[key[q]] + slot[q]] = q;
+}
+
+__global__ void k_pbd_rank(const int32_t* __restrict__ key, const int32_t* __restrict__ start,
+                           const int32_t* __restrict__ list, int32_t* __restrict__ sorted, int32_t n_items,
+                           int32_t per_box) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n_items || key[q] < 0) return;
+  const int b = start[key[q]], e = start[key[q] + 1];
+  int rank = 0;
+  for (int m = b; m < e; ++m) rank += list[m] < q;
+  sorted[b + rank] = q / per_box;
 }
 
 // Collide (:293-351) for the ordered pair (i < j); false when they do not overlap.
@@ -172,12 +170,22 @@ __device__ bool collide(const PbdConst& c, const cwa_pbd_box& bi, const cwa_pbd_
   return true;
 }
 
-// CollisionQuery (:225-290) for box i against the boxes of higher index.
-__global__ void k_pbd_query(PbdConst c, cwa_pbd_box* __restrict__ boxes, const int32_t* __restrict__ cstart,
-                            const int32_t* __restrict__ csorted, PbdPair* __restrict__ pairs,
-                            int32_t* __restrict__ npairs, int32_t* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
+// CollisionQuery (:225-290) for box i against the boxes of higher index, one
+// warp a box.  The cells of a row (ci, cj) are consecutive, so a row's members
+// are one range of the sorted list; the lanes fetch the rows' ranges side by
+// side and test the members of all rows as one sequence, 32 at a time.  A
+// contact's slot is the number of contacts before it in list order, which the
+// ballots give.  A contact enters its higher box's list in arrival order.
+// Latency bounds it (a member costs two dependent loads): one thread a box
+// walked ~100 members in turn on 32 CTAs, 296 us at 4096 boxes; this form
+// takes 26 us (both with cold caches).
+__global__ void __launch_bounds__(128)
+    k_pbd_query(PbdConst c, cwa_pbd_box* __restrict__ boxes, const int32_t* __restrict__ cstart,
+                const int32_t* __restrict__ csorted, PbdPair* __restrict__ pairs, int32_t* __restrict__ npairs,
+                int32_t* __restrict__ rcount, int32_t* __restrict__ rlist, int32_t* status) {
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= c.n) return;  // whole warps leave together
   const cwa_pbd_box bi = boxes[i];
   float qmin[3], qmax[3];
   int lo[3], hi[3];
@@ -188,68 +196,100 @@ __global__ void k_pbd_query(PbdConst c, cwa_pbd_box* __restrict__ boxes, const i
     lo[a] = cell_c(c, qmin[a], a);
     hi[a] = cell_c(c, qmax[a], a);
   }
-  int t = 0;
-  for (int ci = lo[0]; ci <= hi[0]; ++ci)
-    for (int cj = lo[1]; cj <= hi[1]; ++cj)
-      for (int ck = lo[2]; ck <= hi[2]; ++ck) {
-        const int cell = cell_id(c, ci, cj, ck);
-        for (int r = cstart[cell]; r < cstart[cell + 1]; ++r) {
-          const int j = csorted[r] / c.maxc;
-          if (j <= i) continue;  // Collide returns for i >= j
-          const cwa_pbd_box& bj = boxes[j];
-          float bmin[3], bmax[3];
-          int home[3];
+  const float4 red = make_float4(1.0f, 0.0f, 0.0f, 1.0f);
+  const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1, rows = (hi[0] - lo[0] + 1) * ny;
+  int t = 0;  // contacts so far (warp-uniform)
+  for (int row0 = 0; row0 < rows; row0 += 32) {
+    // lane l: row row0 + l, its first cell and its members' range
+    const int nrow = min(rows - row0, 32);
+    int cell0 = 0, first = 0, len = 0;
+    if (lane < nrow) {
+      const int x = (row0 + lane) / ny;
+      cell0 = cell_id(c, lo[0] + x, lo[1] + row0 + lane - x * ny, lo[2]);
+      first = cstart[cell0];
+      len = cstart[cell0 + nz] - first;
+    }
+    int incl = len;
 #pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            bmin[a] = fs(bj.x[a], bj.hw[a]);
-            bmax[a] = fa(bj.x[a], bj.hw[a]);
-            home[a] = max(lo[a], cell_c(c, bmin[a], a));
-          }
-          if (home[0] != ci || home[1] != cj || home[2] != ck) continue;
-          PbdPair pr;
-          if (!collide(c, bi, bj, qmin, qmax, bmin, bmax, &pr)) continue;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int m0 = 0; m0 < total; m0 += 32) {
+      const int m = m0 + lane;
+      int row = 0;  // the member's row: the rows whose ranges end at or before m
+      for (int k = 0; k + 1 < nrow; ++k) row += m >= __shfl_sync(0xffffffffu, incl, k);
+      const int rc = __shfl_sync(0xffffffffu, cell0, row);
+      const int r = m + __shfl_sync(0xffffffffu, first - (incl - len), row);
+      bool hit = false;
+      int j = 0;
+      PbdPair pr;
+      if (m < total && (j = csorted[r]) > i) {  // Collide returns for i >= j
+        int ck = 0;
+        while (r >= cstart[rc + ck + 1]) ++ck;
+        const cwa_pbd_box& bj = boxes[j];
+        float bmin[3], bmax[3];
+        int home[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          bmin[a] = fs(bj.x[a], bj.hw[a]);
+          bmax[a] = fa(bj.x[a], bj.hw[a]);
+          home[a] = max(lo[a], cell_c(c, bmin[a], a));
+        }
+        if (cell_id(c, home[0], home[1], home[2]) == rc + ck)
+          hit = collide(c, bi, bj, qmin, qmax, bmin, bmax, &pr);
+      }
+      const unsigned hits = __ballot_sync(0xffffffffu, hit);
+      if (hit) {
+        const int slot = t + __popc(hits & ((1u << lane) - 1u));
+        if (slot < c.pcap) {
+          const int q = i * c.pcap + slot;
           pr.i = i;
           pr.j = j;
-          if (t < c.pcap)
-            pairs[(size_t)i * c.pcap + t] = pr;
-          else
-            atomicOr(status, kStatusBigCell);
-          ++t;
-          const float red[4] = {1.0f, 0.0f, 0.0f, 1.0f};
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            boxes[i].color[a] = red[a];  // the same value from every writer
-            boxes[j].color[a] = red[a];
-          }
+          pairs[q] = pr;
+          const int s = atomicAdd(rcount + j, 1);
+          if (s < c.pcap) rlist[(size_t)j * c.pcap + s] = q;  // past pcap: the post pass searches the pairs
+        } else {
+          atomicOr(status, kStatusBigCell);
         }
+        // the same value from every writer
+        *reinterpret_cast<float4*>(boxes[i].color) = red;
+        *reinterpret_cast<float4*>(boxes[j].color) = red;
       }
-  npairs[i] = min(t, c.pcap);
-}
-
-// The pairs indexed by their higher box: key = j for the used slots.
-__global__ void k_pbd_rev_key(PbdConst c, const PbdPair* __restrict__ pairs, const int32_t* __restrict__ npairs,
-                              int32_t* __restrict__ rkey, int32_t* __restrict__ rslot, int32_t* __restrict__ rcount) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= c.n * c.pcap) return;
-  const int i = q / c.pcap, t = q - i * c.pcap;
-  if (t >= npairs[i]) {
-    rkey[q] = -1;
-    return;
+      t += __popc(hits);
+    }
   }
-  const int j = pairs[q].j;
-  rkey[q] = j;
-  rslot[q] = count_slot(rcount, j);
+  if (lane == 0) npairs[i] = min(t, c.pcap);
 }
 
-// wall terms, then the own pairs, then the partner pairs; PostAnimate (:372-392)
-__global__ void k_pbd_post(PbdConst c, cwa_pbd_box* __restrict__ boxes, const PbdPair* __restrict__ pairs,
-                           const int32_t* __restrict__ npairs, const int32_t* __restrict__ rstart,
-                           const int32_t* __restrict__ rsorted) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= c.n) return;
-  cwa_pbd_box o = boxes[b];
+// Wall terms, then the own pairs, then the partner pairs; PostAnimate
+// (:372-392).  Eight lanes a box: lane k < 3 sums component k of the normal
+// displacement, lane k + 3 that of the friction, lane 6 counts, each in the
+// fixed order, so a lane's chain is one addition a pair and the pairs' loads
+// are shared by the lanes and run ahead of the sums.  The box's partner list
+// is sorted first (each entry's rank is the number of smaller ones), in shared
+// memory up to kPostList entries; longer lists, rare, are taken smallest entry
+// first, and one past its pcap slots is replaced by a search of all pairs in
+// slot order.  One thread a box took 22 us at 4096 boxes, this
+// form 11 us, and the list replaces a counting sort of all pair slots (a key
+// pass, a scan and two passes over n pcap slots, 19 us).
+constexpr int kPostLanes = 8;
+constexpr int kPostThreads = 128;
+constexpr int kPostList = 64;
+
+__global__ void __launch_bounds__(kPostThreads)
+    k_pbd_post(PbdConst c, cwa_pbd_box* __restrict__ boxes, const PbdPair* __restrict__ pairs,
+               const int32_t* __restrict__ npairs, const int32_t* __restrict__ rcount,
+               const int32_t* __restrict__ rlist) {
+  __shared__ int32_t s_in[kPostThreads / kPostLanes][kPostList], s_out[kPostThreads / kPostLanes][kPostList];
+  const int b = (blockIdx.x * kPostThreads + threadIdx.x) / kPostLanes;
+  const int k = threadIdx.x % kPostLanes, g = threadIdx.x / kPostLanes;
+  const unsigned team = 0xffu << ((threadIdx.x & 31) - k);
+  if (b >= c.n) return;  // whole teams leave together
+  const cwa_pbd_box o = boxes[b];
   float dpn[3] = {0.0f, 0.0f, 0.0f}, dpt[3] = {0.0f, 0.0f, 0.0f}, nn = 0.0f;
-  // collisions with the extents (:230-259)
+  // collisions with the extents (:230-259), on every lane
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float qmin = fs(o.p[a], o.hw[a]), qmax = fa(o.p[a], o.hw[a]);
@@ -270,59 +310,72 @@ __global__ void k_pbd_post(PbdConst c, cwa_pbd_box* __restrict__ boxes, const Pb
       for (int q = 0; q < 3; ++q) dpt[q] = fa(dpt[q], s == 1.0f ? dp[q] : fm(dp[q], s));
     }
   }
-  for (int t = 0; t < npairs[b]; ++t) {  // b is the lower box
-    const PbdPair& pr = pairs[(size_t)b * c.pcap + t];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      dpn[a] = fa(dpn[a], fm(-pr.wi, pr.disp[a]));
-      dpt[a] = fa(dpt[a], fm(-pr.wi, pr.frict[a]));
+  // this lane's component: its sum so far and its value in a pair
+  float sum = k < 3 ? (k == 0 ? dpn[0] : k == 1 ? dpn[1] : dpn[2])
+                    : k < 6 ? (k == 3 ? dpt[0] : k == 4 ? dpt[1] : dpt[2]) : nn;
+  auto add = [&](const PbdPair& pr, bool own) {
+    const float w = own ? -pr.wi : pr.wj;
+    const float v = reinterpret_cast<const float*>(&pr)[4 + min(k, 5)];  // disp, then frict
+    sum = fa(sum, k < 6 ? fm(w, v) : 1.0f);
+  };
+  const int no = npairs[b];
+  const PbdPair* mine = pairs + (size_t)b * c.pcap;
+#pragma unroll 4
+  for (int t = 0; t < no; ++t) add(mine[t], true);  // b is the lower box
+  const int nr = rcount[b];  // b is the higher box
+  if (nr <= kPostList && nr <= c.pcap) {
+    for (int s = k; s < nr; s += kPostLanes) s_in[g][s] = rlist[(size_t)b * c.pcap + s];
+    __syncwarp(team);
+    for (int s = k; s < nr; s += kPostLanes) {
+      const int q = s_in[g][s];
+      int rank = 0;
+      for (int m = 0; m < nr; ++m) rank += s_in[g][m] < q;
+      s_out[g][rank] = q;
     }
-    nn = fa(nn, 1.0f);
-  }
-  for (int r = rstart[b]; r < rstart[b + 1]; ++r) {  // b is the higher box
-    const PbdPair& pr = pairs[rsorted[r]];
+    __syncwarp(team);
+#pragma unroll 4
+    for (int s = 0; s < nr; ++s) add(pairs[s_out[g][s]], false);
+  } else if (nr <= c.pcap) {
+    // entry by entry: the smallest one above the last
+    const int32_t* list = rlist + (size_t)b * c.pcap;
+    int last = -1;
+    for (int s = 0; s < nr; ++s) {
+      int q = 0x7fffffff;
+      for (int m = k; m < nr; m += kPostLanes)
+        if (list[m] > last) q = min(q, list[m]);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      dpn[a] = fa(dpn[a], fm(pr.wj, pr.disp[a]));
-      dpt[a] = fa(dpt[a], fm(pr.wj, pr.frict[a]));
+      for (int x = 1; x < kPostLanes; x <<= 1) q = min(q, __shfl_xor_sync(team, q, x, kPostLanes));
+      add(pairs[q], false);
+      last = q;
     }
-    nn = fa(nn, 1.0f);
+  } else {
+    for (int i = 0; i < b; ++i)
+      for (int t = 0; t < npairs[i]; ++t) {
+        const PbdPair& pr = pairs[(size_t)i * c.pcap + t];
+        if (pr.j == b) add(pr, false);
+      }
   }
-  float p[3], pe[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    p[a] = o.p[a];
-    pe[a] = o.p[a];
-  }
+  nn = __shfl_sync(team, sum, 6, kPostLanes);
+  const int a = k < 3 ? k : 0;
+  const float dn = __shfl_sync(team, sum, a, kPostLanes), dt = __shfl_sync(team, sum, a + 3, kPostLanes);
+  const float op = a == 0 ? o.p[0] : a == 1 ? o.p[1] : o.p[2], ox = a == 0 ? o.x[0] : a == 1 ? o.x[1] : o.x[2];
+  float p = op, pe = op;
   if (nn > 0.0f) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      p[a] = fa(p[a], fd(fm(c.k, fa(dpt[a], dpn[a])), nn));
-      pe[a] = fa(pe[a], fd(fm(c.k, fa(dpt[a], fm(c.e, dpn[a]))), nn));
-      o.p[a] = p[a];
-    }
+    p = fa(p, fd(fm(c.k, fa(dt, dn)), nn));
+    pe = fa(pe, fd(fm(c.k, fa(dt, fm(c.e, dn))), nn));
   }
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    o.v[a] = fd(fs(pe[a], o.x[a]), c.dt);
-    o.dp_n[a] = dpn[a];
-    o.dp_t[a] = dpt[a];
+  const float moved = fs(ox, p);
+  const bool awake = len3(__shfl_sync(team, moved, 0, kPostLanes), __shfl_sync(team, moved, 1, kPostLanes),
+                          __shfl_sync(team, moved, 2, kPostLanes)) > c.sleep;
+  if (k < 3) {
+    cwa_pbd_box& w = boxes[b];
+    w.v[a] = fd(fs(pe, ox), c.dt);
+    w.dp_n[a] = dn;
+    w.dp_t[a] = dt;
+    w.p[a] = p;
+    if (awake) w.x[a] = p;
+    if (a == 0) w.n = nn;
   }
-  o.n = nn;
-  if (len3(fs(o.x[0], p[0]), fs(o.x[1], p[1]), fs(o.x[2], p[2])) > c.sleep)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) o.x[a] = p[a];
-  boxes[b].x[0] = o.x[0];
-  boxes[b].x[1] = o.x[1];
-  boxes[b].x[2] = o.x[2];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    boxes[b].p[a] = o.p[a];
-    boxes[b].v[a] = o.v[a];
-    boxes[b].dp_n[a] = o.dp_n[a];
-    boxes[b].dp_t[a] = o.dp_t[a];
-  }
-  boxes[b].n = o.n;
 }
 
 constexpr int kB = 128;
@@ -342,10 +395,9 @@ struct cwa_pbd_sim {
   int32_t *ikey = nullptr, *islot = nullptr, *ccount = nullptr, *cstart = nullptr, *clist = nullptr,
           *csorted = nullptr;
   PbdPair* pairs = nullptr;
-  int32_t *npairs = nullptr, *rkey = nullptr, *rslot = nullptr, *rcount = nullptr, *rstart = nullptr,
-          *rlist = nullptr, *rsorted = nullptr;
-  void *ws_cells = nullptr, *ws_rev = nullptr;
-  ScanWorkspace scan_cells{}, scan_rev{};
+  int32_t *npairs = nullptr, *rcount = nullptr, *rlist = nullptr;
+  void* ws_cells = nullptr;
+  ScanWorkspace scan_cells{};
   int32_t* d_status = nullptr;
   int ncells = 0;
   bool uploaded = false;
@@ -383,8 +435,8 @@ void free_pbd(cwa_pbd_sim* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->graph) cudaGraphExecDestroy(s->graph);
   free_items(s);
-  void* ps[] = {s->boxes, s->ccount, s->cstart, s->pairs, s->npairs, s->rkey, s->rslot, s->rcount,
-                s->rstart, s->rlist, s->rsorted, s->ws_cells, s->ws_rev, s->d_status};
+  void* ps[] = {s->boxes,  s->ccount, s->cstart,   s->pairs,   s->npairs,
+                s->rcount, s->rlist,  s->ws_cells, s->d_status};
   for (void* p : ps) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
@@ -393,21 +445,16 @@ void free_pbd(cwa_pbd_sim* s) {
 cwa_status enqueue_substep(cwa_pbd_sim* s) {
   const PbdConst& c = s->k;
   cudaStream_t st = s->stream;
-  const long items = (long)c.n * c.maxc, slots = (long)c.n * c.pcap;
-  k_pbd_cells<<<nb(c.n), kB, 0, st>>>(c, s->boxes, s->ikey, s->islot, s->ccount, s->d_status);
+  const long items = (long)c.n * c.maxc;
+  k_pbd_cells<<<nb(items), kB, 0, st>>>(c, s->boxes, s->ikey, s->islot, s->ccount, s->rcount, s->d_status);
   PBD_CUDA(cudaGetLastError());
-  PBD_CUDA(scan_launch(s->ccount, s->cstart, s->ncells, s->ncells + 1, true, s->scan_cells, s->d_status, st,
-                       nullptr));
+  PBD_CUDA(scan_launch_two_pass(s->ccount, s->cstart, s->ncells, s->ncells + 1, true, s->scan_cells, st, nullptr));
   k_pbd_insert<<<nb(items), kB, 0, st>>>(s->ikey, s->islot, s->cstart, s->clist, (int32_t)items);
-  k_pbd_rank<<<nb(items), kB, 0, st>>>(s->ikey, s->cstart, s->clist, s->csorted, (int32_t)items);
-  k_pbd_pre<<<nb(c.n), kB, 0, st>>>(c, s->boxes);
-  k_pbd_query<<<nb(c.n), kB, 0, st>>>(c, s->boxes, s->cstart, s->csorted, s->pairs, s->npairs, s->d_status);
-  k_pbd_rev_key<<<nb(slots), kB, 0, st>>>(c, s->pairs, s->npairs, s->rkey, s->rslot, s->rcount);
-  PBD_CUDA(cudaGetLastError());
-  PBD_CUDA(scan_launch(s->rcount, s->rstart, c.n, c.n + 1, true, s->scan_rev, s->d_status, st, nullptr));
-  k_pbd_insert<<<nb(slots), kB, 0, st>>>(s->rkey, s->rslot, s->rstart, s->rlist, (int32_t)slots);
-  k_pbd_rank<<<nb(slots), kB, 0, st>>>(s->rkey, s->rstart, s->rlist, s->rsorted, (int32_t)slots);
-  k_pbd_post<<<nb(c.n), kB, 0, st>>>(c, s->boxes, s->pairs, s->npairs, s->rstart, s->rsorted);
+  k_pbd_rank<<<nb(items), kB, 0, st>>>(s->ikey, s->cstart, s->clist, s->csorted, (int32_t)items, c.maxc);
+  k_pbd_query<<<nb(32l * c.n), kB, 0, st>>>(c, s->boxes, s->cstart, s->csorted, s->pairs, s->npairs, s->rcount,
+                                            s->rlist, s->d_status);
+  k_pbd_post<<<(unsigned)(((long)c.n * kPostLanes + kPostThreads - 1) / kPostThreads), kPostThreads, 0, st>>>(
+      c, s->boxes, s->pairs, s->npairs, s->rcount, s->rlist);
   PBD_CUDA(cudaGetLastError());
   return CWA_OK;
 }
@@ -476,17 +523,11 @@ cwa_status cwa_pbd_create(const cwa_pbd_params* p, int32_t device, cwa_pbd_sim**
   al((void**)&s->cstart, 4 * ((size_t)s->ncells + 1));
   al((void**)&s->pairs, sizeof(PbdPair) * slots);
   al((void**)&s->npairs, 4 * (size_t)k.n);
-  al((void**)&s->rkey, 4 * slots);
-  al((void**)&s->rslot, 4 * slots);
   al((void**)&s->rlist, 4 * slots);
-  al((void**)&s->rsorted, 4 * slots);
   al((void**)&s->rcount, 4 * (size_t)k.n);
-  al((void**)&s->rstart, 4 * ((size_t)k.n + 1));
   al(&s->ws_cells, scan_workspace_bytes(s->ncells + 1));
-  al(&s->ws_rev, scan_workspace_bytes(k.n + 1));
   al((void**)&s->d_status, 4);
   if (e == cudaSuccess) e = cudaMemset(s->ccount, 0, 4 * (size_t)s->ncells);
-  if (e == cudaSuccess) e = cudaMemset(s->rcount, 0, 4 * (size_t)k.n);
   if (e == cudaSuccess) e = cudaMemset(s->npairs, 0, 4 * (size_t)k.n);
   if (e == cudaSuccess) e = cudaMemset(s->d_status, 0, 4);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
@@ -496,7 +537,6 @@ cwa_status cwa_pbd_create(const cwa_pbd_params* p, int32_t device, cwa_pbd_sim**
     return e == cudaErrorMemoryAllocation ? CWA_ERR_OOM : CWA_ERR_CUDA;
   }
   scan_bind_workspace(s->ws_cells, s->ncells + 1, &s->scan_cells);
-  scan_bind_workspace(s->ws_rev, k.n + 1, &s->scan_rev);
   *out = s;
   return CWA_OK;
 }
@@ -523,11 +563,11 @@ cwa_status cwa_pbd_upload(cwa_pbd_sim* s, const cwa_pbd_box* host, int32_t n) {
   for (int a = 0; a < 3; ++a)
     maxc *= std::min<long>(dims[a], (long)floorf(2.0f * hmax[a] / s->k.cell[a]) + 2);
   if (maxc * n > (1l << 30)) return perr("boxes too large for the grid", CWA_ERR_CAPACITY);
-  if (s->graph) {
-    cudaGraphExecDestroy(s->graph);
-    s->graph = nullptr;
-  }
   if (maxc != s->k.maxc || !s->ikey) {
+    if (s->graph) {  // it holds the old item buffers
+      cudaGraphExecDestroy(s->graph);
+      s->graph = nullptr;
+    }
     free_items(s);
     s->k.maxc = (int)maxc;
     const size_t items = (size_t)maxc * n;
@@ -578,10 +618,12 @@ cwa_status cwa_pbd_step(cwa_pbd_sim* s, int32_t n_steps) {
 cwa_status cwa_pbd_pair_count(cwa_pbd_sim* s, int64_t* pairs) {
   if (!s || !pairs) return perr("null sim or output");
   PBD_CUDA(cudaSetDevice(s->device));
-  int32_t v = 0;
-  PBD_CUDA(cudaMemcpyAsync(&v, s->rstart + s->k.n, 4, cudaMemcpyDeviceToHost, s->stream));
+  std::vector<int32_t> v((size_t)s->k.n);
+  PBD_CUDA(cudaMemcpyAsync(v.data(), s->npairs, 4 * v.size(), cudaMemcpyDeviceToHost, s->stream));
   PBD_CUDA(cudaStreamSynchronize(s->stream));
-  *pairs = v;
+  int64_t total = 0;
+  for (const int32_t x : v) total += x;
+  *pairs = total;
   return read_pbd_status(s);
 }
 
