@@ -83,6 +83,10 @@ struct cwa_sim {
   CUtensorMap* d_wmaps = nullptr;
   WaveBlockTile* d_wbtiles = nullptr;
   int32_t wb_off[kWaveVariants + 1] = {};
+  // variant 0: the strips of K steps a launch are d_strips [strip_off[K],
+  // strip_off[K + 1])
+  WaveStrip* d_strips = nullptr;
+  int32_t strip_off[kWaveStripMaxSteps + 2] = {};
   // work tiles
   Tile* d_ptiles = nullptr;
   int32_t* d_porder = nullptr;  // work-queue order of the particle tiles (capacity porder_cap)
@@ -544,21 +548,48 @@ cwa_status run_wave(cwa_sim* s) {
   return CWA_OK;
 }
 
-// Lazily set up the blocked wave advance: the spare buffer and, for every
-// variant, a tensor map of every scene's field in each of the four buffers
-// and the block tiles.
-cwa_status prepare_wave_blocks(cwa_sim* s) {
-  if (s->d_wbtiles) return CWA_OK;
-  const int nsc = (int)s->sd.size();
+// Lazily set up the wave advance: the spare buffer (shared by every form),
+// the default form's strips, and for the box variants (prepare_wave_boxes) a
+// tensor map of every scene's field in each of the four buffers and the block
+// tiles.
+cwa_status prepare_wave_spare(cwa_sim* s) {
+  if (s->UB[3]) return CWA_OK;
   float* spare = nullptr;
   CWA_TRY(dev_alloc(s, &spare, (size_t)s->w_total));
+  CWA_CUDA(cudaDeviceSynchronize());  // the zero-fill memset ran on the legacy stream
   for (int b = 0; b < 3; ++b) s->UB[b] = s->U[b];
   s->UB[3] = spare;
   for (int b = 0; b < 4; ++b) s->uid[b] = b;
+  return CWA_OK;
+}
+
+cwa_status prepare_wave_strips(cwa_sim* s) {
+  if (s->d_strips) return CWA_OK;
+  CWA_TRY(prepare_wave_spare(s));
+  int sms = 0;
+  CWA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  std::vector<WaveStrip> strips;
+  for (int k = 2; k <= kWaveStripMaxSteps; ++k) {
+    s->strip_off[k] = (int32_t)strips.size();
+    wave_strips(s->sd, k, sms, &strips);
+  }
+  s->strip_off[kWaveStripMaxSteps + 1] = (int32_t)strips.size();
+  WaveStrip* d = nullptr;
+  CWA_TRY(dev_alloc(s, &d, strips.size()));
+  CWA_CUDA(cudaMemcpy(d, strips.data(), strips.size() * sizeof(WaveStrip), cudaMemcpyHostToDevice));
+  CWA_CUDA(cudaDeviceSynchronize());
+  s->d_strips = d;
+  return CWA_OK;
+}
+
+cwa_status prepare_wave_boxes(cwa_sim* s) {
+  if (s->d_wbtiles) return CWA_OK;
+  CWA_TRY(prepare_wave_spare(s));
+  const int nsc = (int)s->sd.size();
   std::vector<CUtensorMap> maps((size_t)kWaveVariants * 4 * nsc);
   memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
   std::vector<WaveBlockTile> tiles;
-  for (int v = 0; v < kWaveVariants; ++v) {
+  for (int v = 1; v < kWaveVariants; ++v) {
     s->wb_off[v] = (int32_t)tiles.size();
     for (int k = 0; k < nsc; ++k) {
       const SceneDev& d = s->sd[k];
@@ -582,11 +613,11 @@ cwa_status prepare_wave_blocks(cwa_sim* s) {
 }
 
 // n wave passes: a single pass first when deposits are pending (it applies
-// and clears them), K-step blocks of the sim's wave_block variant, single
-// passes for the remainder.  A block writes u^(n+K) into the free slot and
-// u^(n+K-1) into the spare; the slots are then renamed so U[wcur] /
-// U[(wcur+2)%3] hold them, which is the state K single passes leave (up to
-// the rotation of wcur).
+// and clears them), launches of K steps of the sim's wave_block variant (the
+// default takes 2 to 8 steps a launch), single passes for the remainder.
+// A launch writes u^(n+K) into the free slot and u^(n+K-1) into the spare; the
+// slots are then renamed so U[wcur] / U[(wcur+2)%3] hold them, which is the
+// state K single passes leave (up to the rotation of wcur).
 cwa_status run_wave_advance(cwa_sim* s, int32_t n) {
   int32_t done = 0;
   bool coupled = false;
@@ -595,33 +626,59 @@ cwa_status run_wave_advance(cwa_sim* s, int32_t n) {
     CWA_TRY(run_wave(s));
     done = 1;
   }
-  const int v = s->opt.wave_block, K = wave_variant_steps(v);
-  if (n - done >= K) {
-    CWA_TRY(prepare_wave_blocks(s));
-    const int w = s->wcur, cur = w, prev = (w + 2) % 3, nxt = (w + 1) % 3;
+  const int v = s->opt.wave_block;
+  const int w = s->wcur, cur = w, prev = (w + 2) % 3, nxt = (w + 1) % 3;
+  auto renamed = [&](int32_t steps) {
+    const int ic = s->uid[cur], ip = s->uid[prev];
+    s->uid[cur] = s->uid[nxt];
+    s->uid[prev] = s->uid[3];
+    s->uid[nxt] = ic;
+    s->uid[3] = ip;
+    done += steps;
+    s->steps += steps;
+  };
+  const int32_t before = done;
+  if (v == 0) {
+    // as few launches as 8 steps each allow, of as equal a number of steps as
+    // possible: a remainder run as 4 + 1 took a third of 773 x 1021's 29 steps
+    if (n - done >= 2) CWA_TRY(prepare_wave_strips(s));
+    for (int32_t left = n - done; left >= 2; left = n - done) {
+      const int32_t launches = (left + kWaveStripMaxSteps - 1) / kWaveStripMaxSteps;
+      const int32_t K = (left + launches - 1) / launches;
+      WaveStripArgs a;
+      a.in_cur = s->UB[s->uid[cur]];
+      a.in_prev = s->UB[s->uid[prev]];
+      a.out_cur = s->UB[s->uid[nxt]];
+      a.out_prev = s->UB[s->uid[3]];
+      a.strips = s->d_strips + s->strip_off[K];
+      a.scenes = s->d_scenes;
+      const int32_t n_strips = s->strip_off[K + 1] - s->strip_off[K];
+      CWA_CUDA(launch_wave_strips(a, n_strips, K, s->stream));
+      s->launches += n_strips > 0;
+      renamed(K);
+    }
+  } else {
+    const int K = wave_variant_steps(v);
+    if (n - done >= K) CWA_TRY(prepare_wave_boxes(s));
     const int32_t n_tiles = s->wb_off[v + 1] - s->wb_off[v];
     while (n - done >= K) {
-      const int ic = s->uid[cur], ip = s->uid[prev], oc = s->uid[nxt], op = s->uid[3];
       const size_t nsc = s->sd.size();
       WaveBlockArgs a;
-      a.in_cur = s->UB[ic];
-      a.in_prev = s->UB[ip];
-      a.out_cur = s->UB[oc];
-      a.out_prev = s->UB[op];
-      a.map_cur = s->d_wmaps + ((size_t)v * 4 + ic) * nsc;
-      a.map_prev = s->d_wmaps + ((size_t)v * 4 + ip) * nsc;
+      a.in_cur = s->UB[s->uid[cur]];
+      a.in_prev = s->UB[s->uid[prev]];
+      a.out_cur = s->UB[s->uid[nxt]];
+      a.out_prev = s->UB[s->uid[3]];
+      a.map_cur = s->d_wmaps + ((size_t)v * 4 + s->uid[cur]) * nsc;
+      a.map_prev = s->d_wmaps + ((size_t)v * 4 + s->uid[prev]) * nsc;
       a.tiles = s->d_wbtiles + s->wb_off[v];
       a.scenes = s->d_scenes;
       a.status = s->d_status;
       CWA_CUDA(launch_wave_block(a, n_tiles, v, s->stream));
       s->launches += n_tiles > 0;
-      s->uid[cur] = oc;
-      s->uid[prev] = op;
-      s->uid[nxt] = ic;
-      s->uid[3] = ip;
-      done += K;
-      s->steps += K;
+      renamed(K);
     }
+  }
+  if (done > before) {
     for (int b = 0; b < 3; ++b) s->U[b] = s->UB[s->uid[b]];
     drop_graphs(s);  // captured steps hold the old buffer pointers
   }
@@ -1551,7 +1608,8 @@ cwa_status cwa_autotune_wave(cwa_sim* s, int32_t trial_steps, cwa_wave_tune_repo
   CWA_TRY(check_sim(s));
   if (trial_steps < 1 || trial_steps > 4096) return arg_error("trial_steps must be in [1, 4096]");
   const int32_t steps = (trial_steps + 7) & ~7;
-  CWA_TRY(prepare_wave_blocks(s));
+  CWA_TRY(prepare_wave_strips(s));
+  CWA_TRY(prepare_wave_boxes(s));
   CWA_CUDA(cudaStreamSynchronize(s->stream));
   const size_t W = (size_t)s->w_total;
   const int w0 = s->wcur;

@@ -255,11 +255,11 @@ cudaError_t launch_totals(const float4* pos, const float4* vel, int32_t poff, in
                           const SceneDev* scenes, int32_t scene, double* out, cudaStream_t stream);
 
 // ---- temporally blocked wave advance (cwa_wave_tma.cu) ----
-// Block variants (box 128 x 32 / K 4, 128 x 64 / K 4, 128 x 64 / K 8, each
-// with the column walk in shared memory or held in registers, and a 256 x 32
-// / K 4 box with column pairs in registers, and a persistent register-column
-// form that prefetches each CTA's next 128 x 32 box): K wave steps per
-// launch, equal to the halo width.
+// Block variants from 1 on (box 128 x 64 / K 4 and K 8 with the column walk in
+// shared memory; 128 x 32 / K 4, 128 x 64 / K 4 and K 8 with it in registers;
+// a 256 x 32 / K 4 box with column pairs in registers; and a persistent
+// register-column form that prefetches each CTA's next 128 x 32 box): K wave
+// steps per launch, equal to the halo width.
 constexpr int kWaveVariants = 8;
 int wave_variant_steps(int variant);
 
@@ -286,6 +286,27 @@ struct WaveBlockArgs {
 bool wave_block_encode(CUtensorMap* map, float* base, int W, int H, int variant);
 void wave_block_tiles(const SceneDev& d, int32_t scene, bool tma, int variant, std::vector<WaveBlockTile>* out);
 cudaError_t launch_wave_block(const WaveBlockArgs& a, int32_t n_tiles, int variant, cudaStream_t stream);
+
+// ---- the wave advance's default form: register strips (cwa_wave_strip.cu) ----
+// A warp's strip: the sx-th of a scene's strips of columns, output rows
+// [row0, row1).
+struct WaveStrip {
+  int32_t scene, sx, row0, row1;
+};
+struct WaveStripArgs {
+  const float* in_cur;   // u^n (all scenes, woff-offset inside)
+  const float* in_prev;  // u^(n-1)
+  float* out_cur;        // receives u^(n+K)
+  float* out_prev;       // receives u^(n+K-1)
+  const WaveStrip* strips;
+  const SceneDev* scenes;
+  float neg_zero = -0.0f;  // see mul2
+};
+constexpr int kWaveStripMinRows = 16;
+constexpr int kWaveStripMaxSteps = 8;  // a launch takes 2 .. 8 steps
+// The strips of every scene for `steps` steps a launch.
+void wave_strips(const std::vector<SceneDev>& scenes, int steps, int sms, std::vector<WaveStrip>* out);
+cudaError_t launch_wave_strips(const WaveStripArgs& a, int32_t n_strips, int steps, cudaStream_t stream);
 
 // ---- headless rendering (cwa_render.cu) ----
 struct RenderMatrices {  // row-major 4x4

@@ -7,9 +7,9 @@
 //
 // One launch covers all scenes through a list of block tiles.  A block tile
 // owns a (128 - 2K) x (BOX_H - 2K) patch of one scene's field and works on a
-// 128 x BOX_H box: the patch plus a K-cell halo.  Three variants exist
-// (BOX_H, K) = (32, 4), (64, 4), (64, 8); the wave tuner times them and keeps
-// the fastest.  Scenes whose row width is a multiple of 4 cells load the box
+// 128 x BOX_H box: the patch plus a K-cell halo, in several variants of BOX_H,
+// K and the walk; the wave tuner times them and the default form
+// (cwa_wave_strip.cu) and keeps the fastest.  Scenes whose row width is a multiple of 4 cells load the box
 // of u^n and u^(n-1) with two 2D TMA copies (cp.async.bulk.tensor, completion
 // counted on an mbarrier; the box's x origin is patch_x - K, a multiple of 4
 // floats = 16 bytes for K = 4 and 8); other widths load it with plain loads.
@@ -18,8 +18,8 @@
 // exact — and the patch of u^(n+K) and u^(n+K-1) is stored with coalesced
 // writes into two buffers that no CTA of this launch reads.  DRAM traffic
 // per cell-step drops from 12 bytes (single step: read u^n, u^(n-1), write
-// u^(n+1)) to 16 x box / (K x patch) bytes: 4.9 for (32, 4), 4.1 for (64, 4),
-// 2.6 for (64, 8).
+// u^(n+1)) to 16 x box / (K x patch) bytes: 4.9 for (BOX_H, K) = (32, 4), 4.1
+// for (64, 4), 2.6 for (64, 8).
 //
 // Each cell runs the single-step kernel's operation sequence with the same
 // clamped (Neumann) neighbour indices, so one launch equals K single wave
@@ -39,7 +39,8 @@ constexpr int kBoxW = 128;               // box width in cells
 constexpr int kWaveTmaThreads = kBoxW;  // one thread per box column
 
 // The block variants the tuner chooses from: box height and steps per launch
-// (= halo).  Output patch (128 - 2K) x (BOX_H - 2K).
+// (= halo).  Output patch (128 - 2K) x (BOX_H - 2K).  Entry 0 stands for the
+// strips, which are no box.
 constexpr int kVarBoxW[kWaveVariants] = {128, 128, 128, 128, 128, 128, 256, 128};
 constexpr int kVarBoxH[kWaveVariants] = {32, 64, 64, 32, 64, 64, 32, 32};
 constexpr int kVarK[kWaveVariants] = {4, 4, 8, 4, 4, 8, 4, 4};
@@ -715,7 +716,7 @@ cudaError_t launch_wave_block(const WaveBlockArgs& a, int32_t n_tiles, int varia
     case 4: return launch_variant<64, 4, kReg>(a, n_tiles, stream);
     case 5: return launch_variant<64, 8, kReg>(a, n_tiles, stream);
     case 6: return launch_variant<32, 4, kPair>(a, n_tiles, stream);
-    default: return launch_variant<32, 4, kShared>(a, n_tiles, stream);
+    default: return cudaErrorInvalidValue;  // variant 0 is the strips (cwa_wave_strip.cu)
   }
 }
 

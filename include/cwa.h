@@ -136,12 +136,14 @@ typedef struct cwa_sim_options {
   int32_t reserved[2];
 } cwa_sim_options;
 
-/* Blocked wave advance variants: box of 128 x H cells (P: 256 x H) advanced
- * K steps per launch in shared memory; the R and P variants hold each
+/* Wave advance variants.  STRIP (the default): warps march up strips of 128
+ * columns held in registers, 2 to 8 steps per launch.  The others: box of
+ * 128 x H cells (P: 256 x H) advanced K steps per launch in shared memory; the R and P variants hold each
  * thread's box column (P: column pair) in registers and exchange only the
  * east / west neighbours through shared memory. */
 enum {
-  CWA_WAVE_BLOCK_32x4 = 0,  /* default: H 32, K 4 */
+  CWA_WAVE_BLOCK_STRIP = 0,
+  CWA_WAVE_BLOCK_32x4 = 0,  /* the default's earlier name */
   CWA_WAVE_BLOCK_64x4 = 1,  /* H 64, K 4 */
   CWA_WAVE_BLOCK_64x8 = 2,  /* H 64, K 8 */
   CWA_WAVE_BLOCK_R32x4 = 3, /* registers, H 32, K 4 */
@@ -271,8 +273,7 @@ cwa_status cwa_pass_wave(cwa_sim* sim);
  * StencilImage2DTripleBuffered.cpp:22-31 and wave_comp.glsl EvolveWave
  * :171-206, one dispatch per step).  Bit-identical to n_steps calls of
  * cwa_pass_wave; deposits pending from an integrate pass land in the first
- * step.  Steps run K at a time in shared memory (TMA-loaded tiles; K from
- * the sim's wave_block option), so device pointers of the wave buffers may
+ * step.  Steps run several per launch (the sim's wave_block option), so device pointers of the wave buffers may
  * change: re-read cwa_get_device_view after it.  Asynchronous. */
 cwa_status cwa_wave_advance(cwa_sim* sim, int32_t n_steps);
 /* Wait for the sim's stream; report a device-side status (timeout, NaN). */
