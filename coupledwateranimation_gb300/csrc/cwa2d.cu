@@ -114,17 +114,115 @@ __device__ __forceinline__ int cell_i(const Sph2dConst& c, float p, int axis) {
 // the grid's extents [0, view] (point_in_aabb, uniform_grid_sph_cs.glsl:19-23,
 // 101-105); the others go to bucket ncx * ncy past the last cell, which no
 // neighbour search visits, so they are invisible, to themselves too.
-__global__ void k2_hash(Sph2dConst c, const float4* __restrict__ pos, int32_t* __restrict__ key,
-                        int32_t* __restrict__ slot, int32_t* __restrict__ count, int32_t* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n) return;
-  const float4 p = pos[i];
-  if (!finite3(make_float4(p.x, p.y, 0.0f, 0.0f))) atomicOr(status, kStatusNonFinite);
+__device__ __forceinline__ int bucket_of(const Sph2dConst& c, float4 p) {
   const bool inside = p.x > 0.0f && p.y > 0.0f && p.x < c.view_w && p.y < c.view_h;
-  const int k = inside ? cell_i(c, p.x, 0) * c.ncy + cell_i(c, p.y, 1)  // Index(i, j) = i * ny + j
-                       : c.ncx * c.ncy;
+  return inside ? cell_i(c, p.x, 0) * c.ncy + cell_i(c, p.y, 1)  // Index(i, j) = i * ny + j
+                : c.ncx * c.ncy;
+}
+
+__device__ __forceinline__ void hash_particle(const Sph2dConst& c, int i, float4 p, int32_t* __restrict__ key,
+                                              int32_t* __restrict__ slot, int32_t* __restrict__ count) {
+  const int k = bucket_of(c, p);
   key[i] = k;
   slot[i] = count_slot(count, k);
+}
+
+__global__ void k2_hash(Sph2dConst c, const float4* __restrict__ pos, int32_t* __restrict__ key,
+                        int32_t* __restrict__ slot, int32_t* __restrict__ count) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < c.n) hash_particle(c, i, pos[i], key, slot, count);
+}
+
+// Small grids: every CTA scans all the counters itself (its own copy of the
+// cells' starts in shared memory, CTA 0 also writes them out) and inserts its
+// particles, so scan and insert are one launch and the scan needs no zeroed
+// workspace.  Launches of 3 to 5 us of latency each made up the grid's time:
+// hash (now in the force pass), the scan's memset, scan, insert and rank took
+// 17.9 us a substep at 4096 particles, this and the rank 8.8 (cold caches).
+// (The whole build in one CTA with shared-memory counters took 20: one SM's
+// issue slots.)
+constexpr int kScanThreads = 256;
+constexpr int kScanMaxCells = 4096;
+
+__global__ void __launch_bounds__(kScanThreads)
+    k2_scan_insert(int n, int nb, const int32_t* __restrict__ count, const int32_t* __restrict__ key,
+                   const int32_t* __restrict__ slot, int32_t* __restrict__ start, int32_t* __restrict__ list) {
+  __shared__ int32_t s_start[kScanMaxCells + kScanThreads];
+  __shared__ int32_t s_warp[kScanThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i = blockIdx.x * kScanThreads + tid;
+  const int my_key = i < n ? key[i] : -1, my_slot = i < n ? slot[i] : 0;
+  const int per = nb / kScanThreads + 1;  // counters a thread: nb + 1 entries, the last reads 0
+  for (int k = tid; k < per * kScanThreads; k += kScanThreads) s_start[k] = k < nb ? count[k] : 0;
+  __syncthreads();
+  int sum = 0;
+  for (int q = 0; q < per; ++q) sum += s_start[tid * per + q];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  int run = incl - sum;
+  for (int w = 0; w < warp; ++w) run += s_warp[w];
+  for (int q = 0; q < per; ++q) {
+    const int x = s_start[tid * per + q];
+    s_start[tid * per + q] = run;
+    run += x;
+  }
+  __syncthreads();
+  if (my_key >= 0) list[s_start[my_key] + my_slot] = i;
+  if (blockIdx.x == 0)
+    for (int k = tid; k <= nb; k += kScanThreads) start[k] = s_start[k];
+}
+
+// Stable rank (members with a smaller index); sorted: the particle of each
+// sorted place; inv: the inverse; psort: the positions in sorted order.  Also
+// clears the counters for the next count.
+__global__ void __launch_bounds__(256)
+    k2_rank(int n, int nb, const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
+            const int32_t* __restrict__ start, const int32_t* __restrict__ list, const float4* __restrict__ pos,
+            int32_t* __restrict__ sorted, int32_t* __restrict__ inv, float4* __restrict__ psort,
+            int32_t* __restrict__ count, int32_t* status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int k = i; k < nb; k += gridDim.x * blockDim.x) count[k] = 0;
+  if (i >= n) return;
+  const int k = key[i], b = start[k], e = start[k + 1];
+  const float4 p = pos[i];
+  if (!finite3(make_float4(p.x, p.y, 0.0f, 0.0f))) atomicOr(status, kStatusNonFinite);
+  int rank = 0;
+  if (e - b > kMaxStableCell) {
+    rank = slot[i];
+    if (rank == 0) atomicOr(status, kStatusBigCell);
+  } else {
+#pragma unroll 8
+    for (int m = b; m < e; ++m) rank += list[m] < i;
+  }
+  sorted[b + rank] = i;
+  inv[i] = b + rank;
+  psort[b + rank] = p;
+}
+
+// psort again, for a second density pass on the same grid.
+__global__ void k2_order(int n, const float4* __restrict__ pos, const int32_t* __restrict__ sorted,
+                         float4* __restrict__ psort) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) psort[k] = pos[sorted[k]];
+}
+
+// Force's neighbour records in sorted order: (x, y, vx, vy) and (pressure,
+// density), for a force pass that no density pass precedes.
+__global__ void k2_records(int n, const float4* __restrict__ pos, const float4* __restrict__ vel,
+                           const float4* __restrict__ acc, const int32_t* __restrict__ sorted,
+                           float4* __restrict__ rec, float2* __restrict__ pr) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int i = sorted[k];
+  const float4 p = pos[i], v = vel[i];
+  rec[k] = make_float4(p.x, p.y, v.x, v.y);
+  pr[k] = make_float2(v.w, acc[i].w);
 }
 
 __device__ __forceinline__ float warp_sum_f(float v) {
@@ -137,19 +235,61 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 // (member k goes to lane k mod 32) and the partial sums meet in a fixed
 // butterfly, so the result does not depend on scheduling.  (A thread per
 // particle walked ~80 candidates through dependent loads: 16 CTAs on a
-// 4096-particle scene, latency bound.)
+// 4096-particle scene, latency bound.)  The members' data lie in sorted order,
+// one load from the cell's start, and the loads of four cells go out together:
+// with an index load before each and one cell after another the passes were a
+// chain of ~12 round trips (density 7.7 us at 4096 particles with cold caches,
+// now 7.4; force 9.1, now 9.1 with the next grid's hash, 7.9 without).
 constexpr int kWarpsPerBlock = 8;
+constexpr int kCellBatch = 4;
 
-// ComputeDensityPressure (:372-479).
+// Calls visit(slot, k) with each member place k of this lane in the cells
+// [x0, x1] x [y0, y1], cell after cell.  fetch(slot, k, valid) is called before
+// for up to kCellBatch cells at a time, where each holds at most 32 members.
+template <class Fetch, class Visit>
+__device__ __forceinline__ void for_members(const Sph2dConst& c, const int32_t* __restrict__ start, int x0, int x1,
+                                            int y0, int y1, int lane, Fetch fetch, Visit visit) {
+  const int ny = y1 - y0 + 1, cells = (x1 - x0 + 1) * ny;
+  for (int q0 = 0; q0 < cells; q0 += kCellBatch) {
+    int b[kCellBatch], e[kCellBatch];
+    bool big = false;
+#pragma unroll
+    for (int u = 0; u < kCellBatch; ++u) {
+      const int q = q0 + u, dx = q / ny, cell = (x0 + dx) * c.ncy + y0 + q - dx * ny;
+      b[u] = q < cells ? start[cell] : 0;
+      e[u] = q < cells ? start[cell + 1] : 0;
+      big |= e[u] - b[u] > 32;
+    }
+    if (!big) {
+#pragma unroll
+      for (int u = 0; u < kCellBatch; ++u) fetch(u, b[u] + lane, b[u] + lane < e[u]);
+#pragma unroll
+      for (int u = 0; u < kCellBatch; ++u)
+        if (b[u] + lane < e[u]) visit(u, b[u] + lane);
+    } else {
+#pragma unroll 1
+      for (int u = 0; u < kCellBatch; ++u)
+        for (int k = b[u] + lane; k < e[u]; k += 32) {
+          fetch(0, k, true);
+          visit(0, k);
+        }
+    }
+  }
+}
+
+// ComputeDensityPressure (:372-479).  Also writes the particle's force records
+// at its sorted place.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     k2_density(Sph2dConst c, const float4* __restrict__ pin, const float4* __restrict__ vin,
                const float4* __restrict__ ain, float4* __restrict__ pout, float4* __restrict__ vout,
-               float4* __restrict__ aout, const int32_t* __restrict__ start, const int32_t* __restrict__ sorted,
+               float4* __restrict__ aout, const int32_t* __restrict__ start, const float4* __restrict__ psort,
+               const int32_t* __restrict__ inv, float4* __restrict__ rec, float2* __restrict__ pr,
                const float4* __restrict__ wave) {
   const int ix = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (ix >= c.n) return;  // whole warps leave together
   float4 p = pin[ix], v = vin[ix], a = ain[ix];
+  const int place = inv[ix];
   float nx, ny, h, xvel;
   wave_normal_height(c, wave, p.x, &nx, &ny, &h, &xvel);
   const float thresh = 0.05f;
@@ -163,57 +303,62 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     v.x -= 1.75f * vn * db.x;
     v.y -= 1.75f * vn * db.y;
   }
-  if (p.y > c.view_h) {
-    if (lane == 0) {
-      pout[ix] = p;
-      vout[ix] = v;
-      aout[ix] = a;
-    }
-    return;
+  if (!(p.y > c.view_h)) {
+    float rho = 0.0f;
+    const int x0 = cell_i(c, p.x - c.H, 0), x1 = cell_i(c, p.x + c.H, 0);
+    const int y0 = cell_i(c, p.y - c.H, 1), y1 = cell_i(c, p.y + c.H, 1);
+    float4 q[kCellBatch];
+    for_members(
+        c, start, x0, x1, y0, y1, lane,
+        [&](int u, int k, bool valid) {
+          if (valid) q[u] = psort[k];
+        },
+        [&](int u, int) {
+          const float rx = p.x - q[u].x, ry = p.y - q[u].y;
+          const float r2 = rx * rx + ry * ry;
+          if (r2 < c.HSQ) rho += w_cubic(c, sqrtf(r2));
+        });
+    rho = warp_sum_f(rho);
+    if (lane != 0) return;
+    rho = c.mass * rho;
+    if (db.z < c.H) rho += c.psi * w_cubic(c, fmaxf(0.0f, db.z + 0.0f * c.R));
+    rho = fmaxf(c.rest, rho);
+    a.w = rho;
+    v.w = c.gas * (powf(rho / c.rest, 3.0f) - 1.0f);  // WeaklyCompressibleStateEqn, gamma 3
   }
-  float rho = 0.0f;
-  const int x0 = cell_i(c, p.x - c.H, 0), x1 = cell_i(c, p.x + c.H, 0);
-  const int y0 = cell_i(c, p.y - c.H, 1), y1 = cell_i(c, p.y + c.H, 1);
-  for (int ci = x0; ci <= x1; ++ci)
-    for (int cj = y0; cj <= y1; ++cj) {
-      const int cell = ci * c.ncy + cj;
-      for (int k = start[cell] + lane; k < start[cell + 1]; k += 32) {
-        const float4 q = pin[sorted[k]];
-        const float rx = p.x - q.x, ry = p.y - q.y;
-        const float r2 = rx * rx + ry * ry;
-        if (r2 < c.HSQ) rho += w_cubic(c, sqrtf(r2));
-      }
-    }
-  rho = warp_sum_f(rho);
   if (lane != 0) return;
-  rho = c.mass * rho;
-  if (db.z < c.H) rho += c.psi * w_cubic(c, fmaxf(0.0f, db.z + 0.0f * c.R));
-  rho = fmaxf(c.rest, rho);
-  a.w = rho;
-  v.w = c.gas * (powf(rho / c.rest, 3.0f) - 1.0f);  // WeaklyCompressibleStateEqn, gamma 3
   pout[ix] = p;
   vout[ix] = v;
   aout[ix] = a;
+  rec[place] = make_float4(p.x, p.y, v.x, v.y);
+  pr[place] = make_float2(v.w, a.w);
 }
 
 // ComputeForces (:482-627), forward Euler at the end; one warp per particle.
+// The particle's new position is hashed and counted for the next grid here.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     k2_force(Sph2dConst c, const float4* __restrict__ pin, const float4* __restrict__ vin,
              const float4* __restrict__ ain, float4* __restrict__ pout, float4* __restrict__ vout,
-             float4* __restrict__ aout, const int32_t* __restrict__ start, const int32_t* __restrict__ sorted,
-             const float4* __restrict__ wave) {
+             float4* __restrict__ aout, const int32_t* __restrict__ start, const int32_t* __restrict__ inv,
+             const float4* __restrict__ rec, const float2* __restrict__ pr, const float4* __restrict__ wave,
+             int32_t* __restrict__ key, int32_t* __restrict__ slot, int32_t* __restrict__ count) {
   const int ix = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (ix >= c.n) return;
   float4 p = pin[ix], v = vin[ix], a = ain[ix];
+  const int place = inv[ix];
   if (p.w == 0.0f) {
     if (lane == 0) {
       pout[ix] = p;
       vout[ix] = v;
       aout[ix] = a;
+      hash_particle(c, ix, p, key, slot, count);
     }
     return;
   }
+  // the field at the particle, ahead of the sums that need it last
+  float nx, ny, h, vx;
+  wave_normal_height(c, wave, p.x, &nx, &ny, &h, &vx);
   const float rho_i = a.w;
   float apx = 0.0f, apy = 0.0f, avx = 0.0f, avy = 0.0f;
   const float c_visc = -c.visc * 8.0f * c.mass;
@@ -221,30 +366,33 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   const float api = v.w / (rho_i * rho_i);
   const int x0 = cell_i(c, p.x - c.H, 0), x1 = cell_i(c, p.x + c.H, 0);
   const int y0 = cell_i(c, p.y - c.H, 1), y1 = cell_i(c, p.y + c.H, 1);
-  for (int ci = x0; ci <= x1; ++ci)
-    for (int cj = y0; cj <= y1; ++cj) {
-      const int cell = ci * c.ncy + cj;
-      for (int k = start[cell] + lane; k < start[cell + 1]; k += 32) {
-        const int jx = sorted[k];
-        if (jx == ix) continue;
-        const float4 q = pin[jx];
-        const float rx = p.x - q.x, ry = p.y - q.y;
+  float4 q[kCellBatch];
+  float2 s[kCellBatch];
+  for_members(
+      c, start, x0, x1, y0, y1, lane,
+      [&](int u, int k, bool valid) {
+        if (valid) {
+          q[u] = rec[k];
+          s[u] = pr[k];
+        }
+      },
+      [&](int u, int k) {
+        if (k == place) return;
+        const float rx = p.x - q[u].x, ry = p.y - q[u].y;
         const float r = sqrtf(rx * rx + ry * ry);
         if (r < c.H && r > 0.0f) {
           const float wg = w_cubic_grad(c, r);
           const float ux = rx / r, uy = ry / r;
-          const float4 vj = vin[jx];
-          const float rho_j = ain[jx].w;
-          const float sp = (api + vj.w / (rho_j * rho_j)) * wg;
+          const float rho_j = s[u].y;
+          const float sp = (api + s[u].x / (rho_j * rho_j)) * wg;
           apx -= sp * ux;
           apy -= sp * uy;
-          const float vxij = v.x - vj.x, vyij = v.y - vj.y;
+          const float vxij = v.x - q[u].z, vyij = v.y - q[u].w;
           const float sv = 1.0f / rho_j * (vxij * rx + vyij * ry) / (r * r + 0.01f * c.HSQ) * wg;
           avx -= sv * ux;
           avy -= sv * uy;
         }
-      }
-    }
+      });
   apx = warp_sum_f(apx);
   apy = warp_sum_f(apy);
   avx = warp_sum_f(avx);
@@ -260,8 +408,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     apx += c.psi * api * wg * -db.x;
     apy += c.psi * api * wg * -db.y;
   }
-  float nx, ny, h, vx;
-  wave_normal_height(c, wave, p.x, &nx, &ny, &h, &vx);
   const float dh = h - c.view_h / 2.0f;
   const float wave_mask = smoothstepf(0.0f, 0.2f, fabsf(vx));
   float dy = p.y - h;
@@ -277,6 +423,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   pout[ix] = p;
   vout[ix] = v;
   aout[ix] = a;
+  hash_particle(c, ix, p, key, slot, count);
 }
 
 // InitParticle / init_grid (:308-333).
@@ -316,12 +463,10 @@ __device__ __forceinline__ float4 load_or_zero(const float4* w, int i, int n) {
   return (i >= 0 && i < n) ? w[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// IterateWave (:119-148) with FreeBC (:157-174).  Phase 0: half-step values
-// (hm, uhm) between cells i and i+1; phase 1: the full step from them.
-__global__ void k2_wave_iter(Sph2dConst c, const float4* __restrict__ in, float4* __restrict__ out, int phase) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// IterateWave (:119-148) with FreeBC (:157-174) for cell i.  Phase 0: half-step
+// values (hm, uhm) between cells i and i+1; phase 1: the full step from them.
+__device__ __forceinline__ void wave2_cell(const Sph2dConst& c, const float4* in, float4* out, int phase, int i) {
   const int n = c.wave_n;
-  if (i >= n) return;
   const float G = 9.8f, lam = c.lambda, dx = c.dx;
   const float hl = __fdiv_rn(lam, 2.0f);
   // flux of (h, uh): uh^2 / h + g h^2 / 2, one rounding per operation
@@ -345,6 +490,11 @@ __global__ void k2_wave_iter(Sph2dConst c, const float4* __restrict__ in, float4
     if (i == 1) out[0] = w;
     if (i == n - 2) out[n - 1] = w;
   }
+}
+
+__global__ void k2_wave_iter(Sph2dConst c, const float4* __restrict__ in, float4* __restrict__ out, int phase) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < c.wave_n) wave2_cell(c, in, out, phase, i);
 }
 
 // Wave1D_cs.glsl (the 2D app's other wave kind), one rounding per operation.
@@ -393,9 +543,8 @@ __global__ void k1_wave_init(Sph2dConst c, const float4* __restrict__ cur, const
 
 // IterateWave (:120-131): w = atten ((2 - 2 lambda - beta) c0 + lambda (e0 + w0)
 // - (1 - beta) c1), then velocity and acceleration, then FreeBC.
-__global__ void k1_wave_iter(Sph2dConst c, const float4* __restrict__ cur, const float4* __restrict__ prev,
-                             float4* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void wave1_cell(const Sph2dConst& c, const float4* cur, const float4* prev, float4* out,
+                                           int i) {
   const int n = c.wave_n;
   if (i >= n || i == 0 || i == n - 1) return;  // FreeBC: cells 0 and n-1 are written by their neighbours
   const float4 c0 = cur[i], c1 = prev[i], e0 = cur[i + 1], w0 = cur[i - 1];
@@ -407,6 +556,40 @@ __global__ void k1_wave_iter(Sph2dConst c, const float4* __restrict__ cur, const
                          step(c0.w, c1.w, e0.w, w0.w));
   w1_vel_acc(w, c0.x, c1.x);
   w1_store_free(out, i, n, w);
+}
+
+__global__ void k1_wave_iter(Sph2dConst c, const float4* __restrict__ cur, const float4* __restrict__ prev,
+                             float4* __restrict__ out) {
+  wave1_cell(c, cur, prev, out, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// All wave substeps of a frame in one CTA, for fields of at most kWaveCells
+// cells: a substep is a barrier instead of a launch (3.7 us each: two of a
+// frame's launches with the shallow-water kind, ten with Wave1D's ten substeps;
+// one launch of this form takes 5.6 us with the shallow-water kind).  w[0..2]: the buffers in the order of
+// the phase w0 = the newest field's index.
+constexpr int kWaveCells = 4096;
+struct WaveBuffers {
+  float4* w[3];
+};
+
+__global__ void __launch_bounds__(1024) k2_wave_frame(Sph2dConst c, WaveBuffers b, int w0, int substeps) {
+  if (c.wave_kind == CWA2D_WAVE_1D) {
+    int cur = w0;
+    for (int s = 0; s < substeps; ++s) {
+      const int nxt = cur == 2 ? 0 : cur + 1, old = nxt == 2 ? 0 : nxt + 1;
+      for (int i = threadIdx.x; i < c.wave_n; i += blockDim.x) wave1_cell(c, b.w[cur], b.w[old], b.w[nxt], i);
+      __syncthreads();
+      cur = nxt;
+    }
+  } else {
+    for (int s = 0; s < substeps; ++s)
+      for (int phase = 0; phase < 2; ++phase) {
+        const int in = w0 ^ phase;
+        for (int i = threadIdx.x; i < c.wave_n; i += blockDim.x) wave2_cell(c, b.w[in], b.w[in ^ 1], phase, i);
+        __syncthreads();
+      }
+  }
 }
 
 constexpr int kBlock = 256;
@@ -429,6 +612,12 @@ struct cwa2d_sim {
   float4* W[3] = {};
   int cur = 0, wcur = 0;
   int32_t *key = nullptr, *slot = nullptr, *count = nullptr, *start = nullptr, *list = nullptr, *sorted = nullptr;
+  // sorted order: each particle's place, the positions, force's records
+  int32_t* inv = nullptr;
+  float4 *psort = nullptr, *rec = nullptr;
+  float2* pr = nullptr;
+  bool psort_fresh = false, rec_fresh = false;
+  bool counts_pending = false;  // the last force pass has hashed and counted the current positions
   void* scan_ws = nullptr;
   ScanWorkspace scan{};
   int32_t* d_status = nullptr;
@@ -472,6 +661,10 @@ void free2d(cwa2d_sim* s) {
   cudaFree(s->start);
   cudaFree(s->list);
   cudaFree(s->sorted);
+  cudaFree(s->inv);
+  cudaFree(s->psort);
+  cudaFree(s->rec);
+  cudaFree(s->pr);
   cudaFree(s->scan_ws);
   cudaFree(s->d_status);
   cudaFree(s->staging);
@@ -479,29 +672,61 @@ void free2d(cwa2d_sim* s) {
   delete s;
 }
 
+// The positions change outside a force pass: drop its counts.
+cwa_status drop_counts(cwa2d_sim* s) {
+  if (s->counts_pending) {
+    CWA2_CUDA(cudaMemsetAsync(s->count, 0, 4 * ((size_t)s->k.ncx * s->k.ncy + 1), s->stream));
+    s->counts_pending = false;
+  }
+  return CWA_OK;
+}
+
 cwa_status pass_grid(cwa2d_sim* s) {
   const Sph2dConst& c = s->k;
   const int nb = c.ncx * c.ncy + 1;  // the cells and the outside bucket
-  k2_hash<<<blocks(c.n), kBlock, 0, s->stream>>>(c, s->P[s->cur], s->key, s->slot, s->count, s->d_status);
+  if (!s->counts_pending) {
+    k2_hash<<<blocks(c.n), kBlock, 0, s->stream>>>(c, s->P[s->cur], s->key, s->slot, s->count);
+    CWA2_CUDA(cudaGetLastError());
+  }
+  s->counts_pending = false;  // the rank pass clears them
+  if (nb <= kScanMaxCells) {
+    k2_scan_insert<<<(unsigned)((c.n + kScanThreads - 1) / kScanThreads), kScanThreads, 0, s->stream>>>(
+        c.n, nb, s->count, s->key, s->slot, s->start, s->list);
+    CWA2_CUDA(cudaGetLastError());
+  } else {
+    CWA2_CUDA(scan_launch_two_pass(s->count, s->start, nb, nb + 1, false, s->scan, s->stream, nullptr));
+    CWA2_CUDA(launch_list_insert(s->key, s->slot, s->start, s->list, c.n, nullptr, s->stream));
+  }
+  k2_rank<<<blocks(c.n), kBlock, 0, s->stream>>>(c.n, nb, s->key, s->slot, s->start, s->list, s->P[s->cur],
+                                                  s->sorted, s->inv, s->psort, s->count, s->d_status);
   CWA2_CUDA(cudaGetLastError());
-  CWA2_CUDA(scan_launch(s->count, s->start, nb, nb + 1, true, s->scan, s->d_status, s->stream, nullptr));
-  CWA2_CUDA(launch_list_insert(s->key, s->slot, s->start, s->list, c.n, nullptr, s->stream));
-  CWA2_CUDA(launch_point_rank(s->key, s->slot, s->start, s->list, c.n, s->sorted, s->d_status, s->stream));
   s->grid_fresh = true;
+  s->psort_fresh = true;
+  s->rec_fresh = false;
   return CWA_OK;
 }
 
 cwa_status pass_sph(cwa2d_sim* s, bool density) {
-  const int a = s->cur, b = a ^ 1;
-  const unsigned grid = (unsigned)((s->k.n + kWarpsPerBlock - 1) / kWarpsPerBlock);
-  if (density)
-    k2_density<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b],
-                                                              s->A[b], s->start, s->sorted, s->W[s->wcur]);
-  else
-    k2_force<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b],
-                                                            s->A[b], s->start, s->sorted, s->W[s->wcur]);
+  const int a = s->cur, b = a ^ 1, n = s->k.n;
+  const unsigned grid = (unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  if (density) {
+    if (!s->psort_fresh)  // a second density pass on the same grid
+      k2_order<<<blocks(n), kBlock, 0, s->stream>>>(n, s->P[a], s->sorted, s->psort);
+    k2_density<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b], s->A[b],
+                                                              s->start, s->psort, s->inv, s->rec, s->pr,
+                                                              s->W[s->wcur]);
+  } else {
+    if (!s->rec_fresh)  // a force pass straight after the grid's
+      k2_records<<<blocks(n), kBlock, 0, s->stream>>>(n, s->P[a], s->V[a], s->A[a], s->sorted, s->rec, s->pr);
+    k2_force<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b], s->A[b],
+                                                            s->start, s->inv, s->rec, s->pr, s->W[s->wcur], s->key,
+                                                            s->slot, s->count);
+    s->counts_pending = true;
+  }
   CWA2_CUDA(cudaGetLastError());
   s->cur = b;  // StencilBuffer::PingPong
+  s->psort_fresh = false;
+  s->rec_fresh = density;
   if (!density) s->grid_fresh = false;
   return CWA_OK;
 }
@@ -541,6 +766,13 @@ cwa_status enqueue_frame(cwa2d_sim* s) {
     if (st == CWA_OK) st = pass_sph(s, true);
     if (st == CWA_OK) st = pass_sph(s, false);
     if (st != CWA_OK) return st;
+  }
+  if (s->k.wave_n <= kWaveCells && s->prm.wave_substeps > 0) {
+    k2_wave_frame<<<1, 1024, 0, s->stream>>>(s->k, WaveBuffers{{s->W[0], s->W[1], s->W[2]}}, s->wcur,
+                                             s->prm.wave_substeps);
+    CWA2_CUDA(cudaGetLastError());
+    if (s->k.wave_kind == CWA2D_WAVE_1D) s->wcur = (s->wcur + s->prm.wave_substeps) % 3;
+    return CWA_OK;
   }
   for (int sub = 0; sub < s->prm.wave_substeps; ++sub) {
     cwa_status st = CWA_OK;
@@ -672,6 +904,10 @@ cwa_status cwa2d_create(const cwa2d_params* p, int32_t device, cwa2d_sim** out) 
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->slot, 4 * (size_t)k.n);
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->list, 4 * (size_t)k.n);
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->sorted, 4 * (size_t)k.n);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&s->inv, 4 * (size_t)k.n);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&s->psort, sizeof(float4) * k.n);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&s->rec, sizeof(float4) * k.n);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&s->pr, sizeof(float2) * k.n);
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->count, 4 * (size_t)nb);
   if (e == cudaSuccess) e = cudaMalloc((void**)&s->start, 4 * ((size_t)nb + 1));
   if (e == cudaSuccess) e = cudaMalloc(&s->scan_ws, scan_workspace_bytes(nb + 1));
@@ -699,6 +935,8 @@ cwa_status cwa2d_destroy(cwa2d_sim* s) {
 
 cwa_status cwa2d_reinit(cwa2d_sim* s) {
   cwa_status st = check2(s);
+  if (st != CWA_OK) return st;
+  st = drop_counts(s);
   if (st != CWA_OK) return st;
   k2_init_particles<<<blocks(s->k.n), kBlock, 0, s->stream>>>(s->k, s->P[s->cur], s->V[s->cur], s->A[s->cur]);
   // ImageStencil::Reinit: MODE_INIT_FIRST + i into the write image, then
@@ -740,6 +978,13 @@ cwa_status cwa2d_step(cwa2d_sim* s, int32_t n) {
     // per substep); the wave phase advances by 0 (shallow water: two passes
     // per substep) or by wave_substeps mod 3 (Wave1D), so frames replay one
     // graph per wave phase.
+    // Frames start at the scan: the counts come from the frame before, or from
+    // this hash after an upload.
+    if (!s->counts_pending && s->prm.sph_substeps > 0) {
+      k2_hash<<<blocks(s->k.n), kBlock, 0, s->stream>>>(s->k, s->P[s->cur], s->key, s->slot, s->count);
+      CWA2_CUDA(cudaGetLastError());
+      s->counts_pending = true;
+    }
     const int cur0 = s->cur, w0 = s->wcur;
     cudaGraphExec_t& ge = s->graph[w0];
     int w1 = w0;
@@ -763,6 +1008,7 @@ cwa_status cwa2d_step(cwa2d_sim* s, int32_t n) {
     CWA2_CUDA(cudaGraphLaunch(ge, s->stream));
     s->wcur = w1;
     s->grid_fresh = false;
+    if (s->prm.sph_substeps > 0) s->counts_pending = true;
   }
   return CWA_OK;
 }
@@ -794,6 +1040,8 @@ cwa_status cwa2d_upload_particles(cwa2d_sim* s, const cwa2d_particle* host, int3
   cwa_status st = check2(s);
   if (st != CWA_OK) return st;
   if (!host || n != s->k.n) return err2("upload size must equal n_particles");
+  st = drop_counts(s);
+  if (st != CWA_OK) return st;
   // host AoS (48 B) -> device SoA through pitched 2D copies
   const size_t es = sizeof(cwa2d_particle);
   CWA2_CUDA(cudaMemcpy2DAsync(s->P[s->cur], 16, &host[0].pos, es, 16, n, cudaMemcpyHostToDevice, s->stream));
