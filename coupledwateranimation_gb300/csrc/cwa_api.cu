@@ -1734,34 +1734,32 @@ cwa_status cwa_grid_build(const float* d_pos4, int32_t n, const float lo[3], flo
   char* w = reinterpret_cast<char*>(d_workspace);
   ScanWorkspace ws;
   scan_bind_workspace(w, nc + 1, &ws);
-  w += up(scan_workspace_bytes(nc + 1));
-  int32_t* count = reinterpret_cast<int32_t*>(w);
-  w += up((size_t)nc * 4);
+  // the status word (cwa_grid_status reads it) is the workspace's first: one
+  // memset clears it with the counters
+  int32_t* status = reinterpret_cast<int32_t*>(w);
+  const size_t counters = up(scan_workspace_bytes(nc + 1));
+  int32_t* count = reinterpret_cast<int32_t*>(w + counters);
+  const size_t cleared = counters + (size_t)nc * 4;
+  w += counters + up((size_t)nc * 4);
   int32_t* key = reinterpret_cast<int32_t*>(w);
   w += up((size_t)n * 4 + 4);
   int32_t* slot = reinterpret_cast<int32_t*>(w);
   w += up((size_t)n * 4 + 4);
   int32_t* list = reinterpret_cast<int32_t*>(w);
-  w += up((size_t)n * 4 + 4);
-  int32_t* status = reinterpret_cast<int32_t*>(w);  // cwa_grid_status reads it
   if (d_cell_of) key = d_cell_of;
   cudaStream_t st = (cudaStream_t)stream;
-  CWA_CUDA(cudaMemsetAsync(count, 0, (size_t)nc * 4, st));
-  CWA_CUDA(cudaMemsetAsync(status, 0, 4, st));
+  CWA_CUDA(cudaMemsetAsync(d_workspace, 0, cleared, st));
   CWA_CUDA(launch_point_hash(reinterpret_cast<const float4*>(d_pos4), n, lo[0], lo[1], lo[2], cell_size, dims[0],
                              dims[1], dims[2], key, slot, count, status, st));
-  CWA_CUDA(scan_launch(count, d_cell_start, nc, nc + 1, false, ws, status, st, nullptr));
+  CWA_CUDA(scan_launch_two_pass(count, d_cell_start, nc, nc + 1, false, ws, st, nullptr));
   CWA_CUDA(launch_list_insert(key, slot, d_cell_start, list, n, nullptr, st));
-  CWA_CUDA(launch_point_rank(key, slot, d_cell_start, list, n, d_sorted_index, status, st));
+  CWA_CUDA(launch_point_rank(key, d_cell_start, list, n, d_sorted_index, status, st));
   return CWA_OK;
 }
 
 cwa_status cwa_grid_status(int32_t n, int32_t n_cells, const void* d_workspace, void* stream) {
   if (n < 0 || n_cells < 1 || !d_workspace) return arg_error("bad arguments");
-  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t off = up(scan_workspace_bytes(n_cells + 1)) + up((size_t)n_cells * 4) + 3 * up((size_t)n * 4 + 4);
-  return read_status_word(reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(d_workspace) + off),
-                          stream);
+  return read_status_word(reinterpret_cast<const int32_t*>(d_workspace), stream);
 }
 
 }  // extern "C"

@@ -49,18 +49,30 @@ __device__ __forceinline__ bool finite3(float4 p) {
   return isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
 }
 
-// Warp-aggregated count: lanes with the same key share one atomicAdd; each
-// lane's slot is its arrival rank within the cell.
+// Warp-aggregated count: a run of neighbouring lanes with the same key shares
+// one atomicAdd; each lane's slot is its arrival rank within the cell.  Runs
+// catch what matters (particles near cell order; equal keys of scattered
+// points are rare in a warp) for a shuffle and a ballot.  The point grid's
+// build of 1,000,003 scattered points / of the same points sorted, 125 a cell:
+// 59 / 50 us with all equal keys grouped by match.any, 48 / 85 with one atomic
+// a point, 41 / 45 with runs (the last with one memset less, ~2 us).
 __device__ __forceinline__ int count_slot(int32_t* count, int key) {
   const unsigned int active = __activemask();
-  const unsigned int peers = __match_any_sync(active, key);
   const int lane = threadIdx.x & 31;
-  const int leader = __ffs(peers) - 1;
-  const int rank = __popc(peers & ((1u << lane) - 1u));
+  const int prev = __shfl_up_sync(active, key, 1);
+  const bool first = lane == 0 || !((active >> (lane - 1)) & 1u) || prev != key;
+  const unsigned int firsts = __ballot_sync(active, first);
+  // the run: from the nearest first at or below this lane to the lane before
+  // the next first or the next inactive lane
+  const int begin = 31 - __clz(firsts & (0xffffffffu >> (31 - lane)));
   int base = 0;
-  if (lane == leader) base = atomicAdd(count + key, __popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  return base + rank;
+  if (first) {
+    const unsigned int stop = (firsts | ~active) & ~(0xffffffffu >> (31 - lane));  // lanes above this one
+    const int end = stop ? __ffs(stop) - 1 : 32;
+    base = atomicAdd(count + key, end - lane);
+  }
+  base = __shfl_sync(active, base, begin);
+  return base + lane - begin;
 }
 
 // texture(wave_tex, uv) with GL_LINEAR / GL_CLAMP_TO_EDGE on an R32F image

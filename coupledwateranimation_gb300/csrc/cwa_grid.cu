@@ -431,14 +431,24 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void k_point_rank(const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
-                             const int32_t* __restrict__ start, const int32_t* __restrict__ list,
-                             int32_t n, int32_t* __restrict__ sorted_index, int32_t* status) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int k = key[i];
-  int b = start[k], e = start[k + 1];
-  sorted_index[b + stable_rank(list, b, e, i, slot[i], status)] = i;
+// One thread a place of the list, not a point: its reads of the list and of the
+// cells' starts and its write then run along memory, and only the key is a
+// gather.  In point order all four were: the build of 1,000,003 scattered
+// points took 67.5 us, with this 59.3; with 125 points a cell 217 and 71.
+__global__ void k_point_rank(const int32_t* __restrict__ key, const int32_t* __restrict__ start,
+                             const int32_t* __restrict__ list, int32_t n, int32_t* __restrict__ sorted_index,
+                             int32_t* status) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  const int i = list[m], k = key[i], b = start[k], e = start[k + 1];
+  int rank = m - b;  // the place's arrival rank is the point's slot
+  if (e - b > kMaxStableCell) {
+    if (rank == 0) atomicOr(status, kStatusBigCell);
+  } else {
+    rank = 0;
+    for (int q = b; q < e; ++q) rank += list[q] < i;
+  }
+  sorted_index[b + rank] = i;
 }
 
 inline int blocks_for(long n, int b) { return (int)((n + b - 1) / b); }
@@ -561,11 +571,10 @@ cudaError_t launch_point_hash(const float4* pos, int32_t n, float lx, float ly, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_point_rank(const int32_t* key, const int32_t* slot, const int32_t* start,
-                              const int32_t* list, int32_t n, int32_t* sorted_index, int32_t* status,
-                              cudaStream_t stream) {
+cudaError_t launch_point_rank(const int32_t* key, const int32_t* start, const int32_t* list, int32_t n,
+                              int32_t* sorted_index, int32_t* status, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  k_point_rank<<<blocks_for(n, 256), 256, 0, stream>>>(key, slot, start, list, n, sorted_index, status);
+  k_point_rank<<<blocks_for(n, 256), 256, 0, stream>>>(key, start, list, n, sorted_index, status);
   return cudaGetLastError();
 }
 

@@ -154,9 +154,8 @@ cudaError_t launch_copy_back(const float4* p2, const float4* v2, const float4* f
 cudaError_t launch_point_hash(const float4* pos, int32_t n, float lx, float ly, float lz, float cell,
                               int32_t dx, int32_t dy, int32_t dz, int32_t* key, int32_t* slot,
                               int32_t* count, int32_t* status, cudaStream_t stream);
-cudaError_t launch_point_rank(const int32_t* key, const int32_t* slot, const int32_t* start,
-                              const int32_t* list, int32_t n, int32_t* sorted_index, int32_t* status,
-                              cudaStream_t stream);
+cudaError_t launch_point_rank(const int32_t* key, const int32_t* start, const int32_t* list, int32_t n,
+                              int32_t* sorted_index, int32_t* status, cudaStream_t stream);
 
 // ---- SPH kernels (cwa_sph.cu) ----
 // This step's hits (r < h, the particle itself included), written by the
