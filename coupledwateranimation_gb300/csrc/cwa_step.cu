@@ -7,6 +7,8 @@
 // the CPU reproduces them bit for bit, deposits included.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "cwa_device.cuh"
 #include "cwa_internal.h"
 
@@ -269,36 +271,76 @@ __global__ void k_wave_init(float* __restrict__ u, int32_t nx, int32_t nz, float
   u[c] = fmul(peak, sm);
 }
 
-// One thread a 16-byte quarter of a record: a warp reads 512 contiguous
-// bytes (8 records) of the source, which may be page-locked host memory
-// read over the host link, and writes each quarter's 8 words to its array as
-// 128 contiguous bytes.
-__global__ void k_unpack(const float4* __restrict__ aos, int32_t n, int32_t poff, float4* __restrict__ pos,
-                         float4* __restrict__ vel, float4* __restrict__ force, float2* __restrict__ rho_p,
-                         float2* __restrict__ extra, int32_t* __restrict__ id) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= 4L * n) return;
-  const int i = (int)(t >> 2), q = (int)(t & 3);
-  const float4 v = aos[t];
-  if (q == 3) {
-    rho_p[poff + i] = make_float2(v.x, v.y);
-    extra[poff + i] = make_float2(v.z, v.w);
-    id[poff + i] = i;
-  } else {
-    (q == 0 ? pos : q == 1 ? vel : force)[poff + i] = v;
+// 16-byte words a thread keeps in flight in the upload and copy kernels, whose
+// source or destination may be page-locked host memory across the host link.
+// The link, not the SMs, bounds them: kLinkCtas CTAs with deep loads move as
+// much as one thread a word (192 GB/s up, 174 down; 16 CTAs 186 up), and leave
+// the SMs to the kernels of other streams: upload and ten steps of 1M
+// particles with three sims interleaved took 4000 us with the wide grid, 3927
+// with 304 CTAs, 3695 with these.
+constexpr int kLinkDepth = 8;
+constexpr int kLinkThreads = 256;
+constexpr int kLinkCtas = 32;
+// Up to 4 MB latency counts (a transfer takes ~20 us and the host waits for
+// it): one word a thread, and few registers, so that a CTA finds a place beside
+// other streams' kernels sooner.
+constexpr long kLinkSmallWords = 1l << 18;
+
+// A warp reads 512 contiguous bytes (8 records' 16-byte quarters) of the source
+// and writes each quarter's 8 words to its array as 128 contiguous bytes.
+template <int kDepth>
+__global__ void __launch_bounds__(kLinkThreads)
+    k_unpack(const float4* __restrict__ aos, int32_t n, int32_t poff, float4* __restrict__ pos,
+             float4* __restrict__ vel, float4* __restrict__ force, float2* __restrict__ rho_p,
+             float2* __restrict__ extra, int32_t* __restrict__ id) {
+  const long words = 4L * n, stride = (long)gridDim.x * kLinkThreads;  // a multiple of 4: a thread keeps its quarter
+  const int q = threadIdx.x & 3;
+  float4* const out = q == 0 ? pos : q == 1 ? vel : force;
+  for (long t = blockIdx.x * (long)kLinkThreads + threadIdx.x; t < words; t += kDepth * stride) {
+    float4 v[kDepth];
+#pragma unroll
+    for (int u = 0; u < kDepth; ++u)
+      if (t + u * stride < words) v[u] = aos[t + u * stride];
+#pragma unroll
+    for (int u = 0; u < kDepth; ++u) {
+      if (t + u * stride >= words) break;
+      const int i = (int)((t + u * stride) >> 2);
+      if (q == 3) {
+        rho_p[poff + i] = make_float2(v[u].x, v[u].y);
+        extra[poff + i] = make_float2(v[u].z, v[u].w);
+        id[poff + i] = i;
+      } else {
+        out[poff + i] = v[u];
+      }
+    }
   }
 }
 
 // Contiguous copy of n floats, both pointers 16-byte aligned, either side
-// device memory or page-locked host memory: one 16-byte word a thread, and
-// the thread past the last whole word copies the 0-3 floats left.
-__global__ void k_copy_f32(const float* __restrict__ src, float* __restrict__ dst, long n) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long n4 = n >> 2;
-  if (t < n4)
-    reinterpret_cast<float4*>(dst)[t] = reinterpret_cast<const float4*>(src)[t];
-  else if (t == n4)
-    for (long k = n4 * 4; k < n; ++k) dst[k] = src[k];
+// device memory or page-locked host memory: 16-byte words, then the 0-3 floats
+// left.
+template <int kDepth>
+__global__ void __launch_bounds__(kLinkThreads)
+    k_copy_f32(const float* __restrict__ src, float* __restrict__ dst, long n) {
+  const long n4 = n >> 2, stride = (long)gridDim.x * kLinkThreads;
+  const long first = blockIdx.x * (long)kLinkThreads + threadIdx.x;
+  const float4* s4 = reinterpret_cast<const float4*>(src);
+  float4* d4 = reinterpret_cast<float4*>(dst);
+  for (long t = first; t < n4; t += kDepth * stride) {
+    float4 v[kDepth];
+#pragma unroll
+    for (int u = 0; u < kDepth; ++u)
+      if (t + u * stride < n4) v[u] = s4[t + u * stride];
+#pragma unroll
+    for (int u = 0; u < kDepth; ++u)
+      if (t + u * stride < n4) d4[t + u * stride] = v[u];
+  }
+  if (first < (n & 3)) dst[n4 * 4 + first] = src[n4 * 4 + first];
+}
+
+inline unsigned link_grid(long words) {
+  const long wide = (words + kLinkThreads - 1) / kLinkThreads;
+  return (unsigned)(words <= kLinkSmallWords ? wide : std::min(wide, (long)kLinkCtas));
 }
 
 __global__ void k_pack(cwa_particle* __restrict__ aos, int32_t n, int32_t poff, const float4* __restrict__ pos,
@@ -425,15 +467,18 @@ cudaError_t launch_wave_init(float* u, int32_t nx, int32_t nz, float mode, cudaS
 cudaError_t launch_unpack(const cwa_particle* aos, int32_t n, int32_t poff, float4* pos, float4* vel,
                           float4* force, float2* rho_p, float2* extra, int32_t* id, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  k_unpack<<<blocks_for(4L * n, 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(aos), n, poff, pos, vel,
-                                                         force, rho_p, extra, id);
+  auto kern = 4L * n <= kLinkSmallWords ? k_unpack<1> : k_unpack<kLinkDepth>;
+  kern<<<link_grid(4L * n), kLinkThreads, 0, stream>>>(reinterpret_cast<const float4*>(aos), n, poff, pos, vel, force,
+                                                       rho_p, extra, id);
   return cudaGetLastError();
 }
 
 cudaError_t launch_copy_f32(const float* src, float* dst, long n, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) return cudaErrorInvalidValue;
-  k_copy_f32<<<blocks_for((n >> 2) + 1, 256), 256, 0, stream>>>(src, dst, n);
+  const long words = (n >> 2) + 1;
+  auto kern = words <= kLinkSmallWords ? k_copy_f32<1> : k_copy_f32<kLinkDepth>;
+  kern<<<link_grid(words), kLinkThreads, 0, stream>>>(src, dst, n);
   return cudaGetLastError();
 }
 
