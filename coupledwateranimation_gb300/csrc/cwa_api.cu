@@ -652,6 +652,8 @@ cwa_status run_wave_advance(cwa_sim* s, int32_t n) {
       a.out_prev = s->UB[s->uid[3]];
       a.strips = s->d_strips + s->strip_off[K];
       a.scenes = s->d_scenes;
+      a.whole = 1;
+      for (const SceneDev& d : s->sd) a.whole &= d.nx % 4 == 0;
       const int32_t n_strips = s->strip_off[K + 1] - s->strip_off[K];
       CWA_CUDA(launch_wave_strips(a, n_strips, K, s->stream));
       s->launches += n_strips > 0;

@@ -299,6 +299,7 @@ struct WaveStripArgs {
   float* out_prev;       // receives u^(n+K-1)
   const WaveStrip* strips;
   const SceneDev* scenes;
+  int32_t whole;           // every scene's width is a multiple of 4
   float neg_zero = -0.0f;  // see mul2
 };
 constexpr int kWaveStripMinRows = 16;

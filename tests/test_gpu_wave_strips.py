@@ -40,6 +40,17 @@ def test_strip_edges(lib, nx, nz):
     _same([small_muller((3, 3, 3), 0.03, (nx, nz), seed=nx + nz)], 15)
 
 
+@pytest.mark.parametrize("nx", [123, 127, 128, 129, 130, 131, 136, 239, 240, 242, 243, 249, 351, 353])
+@pytest.mark.parametrize("n", [8, 4])  # 8 and 4 columns of halo
+def test_first_and_last_strip(lib, nx, n):
+    _same([small_muller((3, 3, 3), 0.03, (nx, 37), seed=nx)], n)
+
+
+@pytest.mark.parametrize("widths", [(128, 64), (130, 64), (64, 131, 252)])  # of four, and mixed, in one launch
+def test_widths_of_a_batch(lib, widths):
+    _same([small_muller((3, 3, 3), 0.03, (nx, 40), seed=nx) for nx in widths], 8)
+
+
 @pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 8, 9, 23])
 @pytest.mark.parametrize("atten", [1.0, 0.97])
 def test_steps_and_damping(lib, n, atten):
