@@ -131,7 +131,8 @@ __device__ __forceinline__ bool row_valid(const SceneDev* S, CellCoord c, int r)
 }
 
 __device__ __forceinline__ int row_id(const SceneDev* S, CellCoord c, int r) {
-  return S->coff + ((c.x + r / 3 - 1) * S->dims[1] + (c.y + r % 3 - 1)) * S->dims[2];
+  const int nz = S->dims[2], nyz = S->dims[1] * nz;
+  return S->coff + c.x * nyz + c.y * nz + (r / 3 - 1) * nyz + (r % 3 - 1) * nz;
 }
 
 // Cell-based start of each row: the base that row-mask bits and Verlet codes are relative
@@ -150,34 +151,47 @@ __device__ __forceinline__ void row_bases(const SceneDev* S, const int32_t* __re
 // radius carries a 2^-10 margin (about h / 1024 of slack in the window), so
 // neither float rounding nor the approximate square root t * rsqrt(t)
 // (relative error ~1e-7) ever drops a pair.
+//
+// An out-of-domain column is infinitely far, so one comparison rules out
+// either kind of row.  Nine windows a particle are a fifth of the density
+// pass's instructions, so each is kept short: one conversion that rounds down
+// a bound, no scaling around the square root.
 struct RowWindows {
   float dxm, dxp, dym, dyp, zl, izc, zmax, rad2;
   __device__ __forceinline__ RowWindows(const SceneDev* S, float4 p, CellCoord c, float r2) {
     const float x0f = S->lo[0] + (float)c.x * S->cell;
     const float y0f = S->lo[1] + (float)c.y * S->cell;
-    dxm = fmaxf(p.x - x0f, 0.0f);
-    dxp = fmaxf(x0f + S->cell - p.x, 0.0f);
-    dym = fmaxf(p.y - y0f, 0.0f);
-    dyp = fmaxf(y0f + S->cell - p.y, 0.0f);
+    const float far = __int_as_float(0x7f800000);
+    dxm = c.x > 0 ? fmaxf(p.x - x0f, 0.0f) : far;
+    dxp = c.x + 1 < S->dims[0] ? fmaxf(x0f + S->cell - p.x, 0.0f) : far;
+    dym = c.y > 0 ? fmaxf(p.y - y0f, 0.0f) : far;
+    dyp = c.y + 1 < S->dims[1] ? fmaxf(y0f + S->cell - p.y, 0.0f) : far;
     zl = p.z - S->lo[2];
     izc = S->inv_cellz;
     zmax = (float)(S->dims[2] - 1);
     rad2 = r2;
+  }
+  // the z cell of height z over the grid's lowest, clamped to the grid
+  __device__ __forceinline__ int zcell(float z) const {
+    return __float2int_rd(fminf(fmaxf(__fmul_rn(z, izc), 0.0f), zmax));
   }
   __device__ __forceinline__ void range(const SceneDev* S, const int32_t* __restrict__ start, CellCoord c, int r,
                                         int& b, int& e) const {
     const int dx = r / 3 - 1, dy = r % 3 - 1;
     const float ddx = dx < 0 ? dxm : (dx > 0 ? dxp : 0.0f);
     const float ddy = dy < 0 ? dym : (dy > 0 ? dyp : 0.0f);
-    const float d2 = ddx * ddx + ddy * ddy;
-    const bool ok = row_valid(S, c, r) && d2 < rad2;
-    const float t = fmaxf(rad2 - d2, 0.0f);
-    const float w = ok ? t * rsqrtf(t) : 0.0f;  // ok implies t > 0
-    const int z0 = (int)fminf(fmaxf(floorf((zl - w) * izc), 0.0f), zmax);
-    const int z1 = (int)fminf(fmaxf(floorf((zl + w) * izc), 0.0f), zmax);
+    const float d2 = __fmaf_rn(ddx, ddx, __fmul_rn(ddy, ddy));
+    const bool ok = d2 < rad2;
+    const float t = fmaxf(__fsub_rn(rad2, d2), 1e-30f);
+    float w;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(t));
+    w = __fmul_rn(t, w);
     const int row = row_id(S, c, r);
-    b = ok ? __ldg(start + row + z0) : 0;
-    e = ok ? __ldg(start + row + z1 + 1) : 0;
+    b = e = 0;
+    if (ok) {
+      b = __ldg(start + (row + zcell(__fsub_rn(zl, w))));
+      e = __ldg(start + (row + zcell(__fadd_rn(zl, w)) + 1));
+    }
   }
 };
 
@@ -289,7 +303,9 @@ __device__ __forceinline__ uint32_t code_pair(const uint16_t* __restrict__ list,
 
 struct StagePlan {
   int32_t seg_b[kMaxSegs];        // global sorted index of each staged segment
-  int32_t seg_off[kMaxSegs + 1];  // staged offset (prefix of lengths)
+  int32_t seg_len[kMaxSegs];
+  int32_t seg_off[kMaxSegs + 1];  // staged offset (prefix of the lengths rounded up to pairs)
+  int32_t copied;                 // candidates copied: the sum of the lengths
   int32_t seg_delta[kMaxSegs];    // seg_off - seg_b: a staged candidate sits at its sorted index + delta
   int32_t col0;                   // first column (x*ny + y) of the CTA
   int32_t ncols;                  // 1 .. kMaxCols; 0 = read from global memory
@@ -321,20 +337,24 @@ __device__ __forceinline__ void plan_stage(const SceneDev* S, const int32_t* __r
       len = __ldg(start + row + zhi + 1) - gb;
     }
   }
-  int incl = len;
+  const int padded = (len + 1) & ~1;
+  int incl = padded;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int copied = __reduce_add_sync(0xffffffffu, len);
   if (lane < kMaxSegs) {
     sp.seg_b[lane] = gb;
-    sp.seg_off[lane] = incl - len;
-    sp.seg_delta[lane] = incl - len - gb;
+    sp.seg_len[lane] = len;
+    sp.seg_off[lane] = incl - padded;
+    sp.seg_delta[lane] = incl - padded - gb;
   }
   if (lane == 0) {
     sp.seg_off[kMaxSegs] = total;
+    sp.copied = copied;
     sp.col0 = colA;
     sp.ncols = (ncols <= kMaxCols && total <= kStageCap) ? ncols : 0;
   }
@@ -458,6 +478,104 @@ __device__ __forceinline__ double scan_row_fp64(Load load, int len, float4 pi, d
   return part;
 }
 
+// ---- staged candidates in pairs ----
+// The packed float instructions work on two candidates at once and round each
+// like the scalar ones, so the stage is rewritten in place: 24 bytes a pair,
+// (x0, x1), (y0, y1), (z0, z1).
+typedef unsigned long long F2;
+constexpr uint32_t kPairBytes = 24;
+
+// Two pairs a thread and round: a round reads 64 bytes a thread and writes 48,
+// all of them where this or an earlier round has read.
+__device__ __forceinline__ void pair_stage(float4* cand, int pairs) {
+  float2* const out = reinterpret_cast<float2*>(cand);
+#pragma unroll 1
+  for (int q0 = 0; q0 < pairs; q0 += 2 * blockDim.x) {
+    float4 a[2], b[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = q0 + k * blockDim.x + threadIdx.x;
+      if (q < pairs) a[k] = cand[2 * q], b[k] = cand[2 * q + 1];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = q0 + k * blockDim.x + threadIdx.x;
+      if (q < pairs) {
+        out[3 * q] = make_float2(a[k].x, b[k].x);
+        out[3 * q + 1] = make_float2(a[k].y, b[k].y);
+        out[3 * q + 2] = make_float2(a[k].z, b[k].z);
+      }
+    }
+  }
+  // a later tile's bulk copies write the same words
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// scan_row_bits over staged candidates [o0, o0 + len) of the stage at `stage`,
+// in whole pairs: what the first and the last pair may hold besides (a row's
+// candidate outside the window, or the filler) is out of reach.  The distance
+// is formed with its sign turned, nq = r^2 - h^2, so that a hit is a set sign
+// bit (zeros of an exact cancellation are +0 and the GPU's NaNs have none) and
+// goes into the mask with one funnel shift, and min(nq, 0) is what a hit adds
+// and nothing for a miss: 17 instructions a pair in place of 26, and the same
+// bits.
+__device__ __forceinline__ float scan_row_pairs(uint32_t stage, int o0, int len, float4 p, float h, RowMask& bits) {
+  const F2 px = f2(p.x, p.x), py = f2(p.y, p.y), pz = f2(p.z, p.z), minus = f2(-1.0f, -1.0f);
+  const float nh = -(h * h);
+  const F2 nh2 = f2(nh, nh);
+  const int odd = o0 & 1;
+  uint32_t a = stage + kPairBytes * (uint32_t)(o0 >> 1);
+  int left = (len + odd + 1) >> 1;
+  float part = 0.0f;
+  uint32_t lo = 0u, hi = 0u, top = 0u;
+  for (int c0 = 0; left > 0; c0 += 32, left -= 16) {
+    const int n = min(left, 16);
+    uint32_t m = 0u;
+    const uint32_t end = a + kPairBytes * (uint32_t)n;
+#pragma unroll 2
+    for (; a < end; a += kPairBytes) {
+      F2 xj, yj, zj;
+      asm("ld.shared.b64 %0, [%1];" : "=l"(xj) : "r"(a));
+      asm("ld.shared.b64 %0, [%1];" : "=l"(yj) : "r"(a + 8u));
+      asm("ld.shared.b64 %0, [%1];" : "=l"(zj) : "r"(a + 16u));
+      const F2 dx = f2_fma(xj, minus, px), dy = f2_fma(yj, minus, py), dz = f2_fma(zj, minus, pz);
+      const float2 nq = f2_get(f2_fma(dz, dz, f2_fma(dy, dy, f2_fma(dx, dx, nh2))));
+      m = __funnelshift_l(__float_as_uint(nq.x), m, 1);
+      m = __funnelshift_l(__float_as_uint(nq.y), m, 1);
+      const float t0 = fminf(nq.x, 0.0f), t1 = fminf(nq.y, 0.0f);
+      part = fmaf(t0 * t0, -t0, part);
+      part = fmaf(t1 * t1, -t1, part);
+    }
+    m = __brev(m) >> (32 - 2 * n);
+    if (c0 == 0)
+      lo = m;
+    else if (c0 == 32)
+      hi = m;
+    else if (c0 == 64)
+      top = m;
+  }
+  bits = ((RowMask)hi << 32) | lo;
+  if (odd) bits = (bits >> 1) | ((RowMask)top << 63);
+  return part;
+}
+
 // One candidate row in the precision P (hit2 = h^2, rad2 >= its float
 // rounding with a margin).
 template <int P, int U, class Load>
@@ -505,6 +623,7 @@ __device__ __forceinline__ int scan_tile(
   // The list build (rare: Verlet rebuilds only) reads candidates from global
   // memory, which keeps its static shared memory under 48 KB.
   constexpr bool kCanStage = ScanShared<MODE>::kCanStage;
+  constexpr bool kPairs = kCanStage && P != CWA_PREC_FP64;  // the stage is rewritten in pairs (scan_row_pairs)
   float4* const s_cand = sh.cand;
   StagePlan& sp = sh.sp;
   const SceneDev* S = scenes + tl.scene;
@@ -514,11 +633,14 @@ __device__ __forceinline__ int scan_tile(
   if (staged && threadIdx.x < 32) {
     // thread 0 arms the barrier with the stage's bytes, then lane s issues
     // segment s's copy (at most 27 segments: one warp issues them all at once)
-    if (threadIdx.x == 0) mbar_expect_tx(&sh.bar, (uint32_t)sp.seg_off[kMaxSegs] * 16u);
+    if (threadIdx.x == 0) mbar_expect_tx(&sh.bar, (uint32_t)sp.copied * 16u);
     __syncwarp();
     const int s = threadIdx.x;
     if (s < 9 * sp.ncols) {
-      const int len = sp.seg_off[s + 1] - sp.seg_off[s];
+      const int len = sp.seg_len[s];
+      // an odd segment's last pair is filled up with a candidate out of reach
+      const float far = __int_as_float(0x7f800000);
+      if (kPairs && (len & 1)) s_cand[sp.seg_off[s] + len] = make_float4(far, far, far, 0.0f);
       if (len > 0) bulk_g2s(&s_cand[sp.seg_off[s]], pos + sp.seg_b[s], (uint32_t)len * 16u, &sh.bar);
     }
   }
@@ -529,6 +651,10 @@ __device__ __forceinline__ int scan_tile(
     mbar_wait_bounded(&sh.bar, parity);  // let copies in flight land before the CTA moves on
   }
   const int used = (staged ? 1 : 0) | (ready ? 0 : 2);
+  if (kPairs && staged) {
+    pair_stage(s_cand, sp.seg_off[kMaxSegs] >> 1);
+    __syncthreads();
+  }
   const int i = tl.begin + threadIdx.x;
   if (i >= tl.end || !ready) return used;
 
@@ -560,48 +686,67 @@ __device__ __forceinline__ int scan_tile(
       for (int r = 0; r < 9; ++r) base[r] = b[r];
     }
   }
+  // One row's hits as bits relative to the row's base, and its sum.
+  auto row_done = [&](int r, int off0, int len, RowMask bits, T part) {
+    overflow |= off0 + len > kMaskBits;
+    const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
+    // every row is stored (whole sectors: skipping the zero rows would make
+    // each store a partial-sector write that DRAM reads back to merge);
+    // force reads only the rows the bitmap names
+    masks[(size_t)r * n_total + i] = m;
+    if (m != 0u) hits |= 1 << r;
+    acc.add(part);
+  };
+  if (MODE == MODE_DENSITY && staged) {
 #pragma unroll
-  for (int r = 0; r < 9; ++r) {
-    int len = e[r] - b[r];
-    if (CWA_DCHECK_FAILED(len == 0 || (b[r] >= 0 && len > 0 && e[r] <= n_total), status)) len = 0;
-    const int off0 = b[r] - base[r];
-    const float4* cand = pos + b[r];
-    bool in_stage = staged && len > 0;
-    if (in_stage) {
+    for (int r = 0; r < 9; ++r) {
+      int len = e[r] - b[r];
       const int so = b[r] + sp.seg_delta[g * 9 + r];
-      if (CWA_DCHECK_FAILED(g >= 0 && g < sp.ncols && so >= 0 && so + len <= sp.seg_off[kMaxSegs], status))
+      if (CWA_DCHECK_FAILED(len == 0 || (g >= 0 && g < sp.ncols && so >= 0 && so + len <= sp.seg_off[kMaxSegs]),
+                            status))
         len = 0;
-      cand = s_cand + so;
-    }
-    if (MODE == MODE_DENSITY) {
-      // row r's hits as bits relative to the row's cell-based start
       RowMask bits = 0u;
       T part = (T)0;
       if (len > 0) {
-        if (in_stage) {
-          const uint32_t a0 = smem_u32(cand);
+        if (kPairs) {
+          part = scan_row_pairs(smem_u32(s_cand), so, len, pi, S->h, bits);
+        } else {
+          const uint32_t a0 = smem_u32(s_cand + so);
           part = scan_row_prec<P, 2>([&](int o) { return lds128(a0 + 16u * (uint32_t)o); }, len, pi, hit2, S->hs2,
                                      bits);
-        } else
-          part = scan_row_prec<P, 2>([&](int o) { return __ldg(cand + o); }, len, pi, hit2, S->hs2, bits);
+        }
       }
-      overflow |= off0 + len > kMaskBits;
-      const RowMask m = off0 < kMaskBits ? bits << off0 : 0u;
-      // every row is stored (whole sectors: skipping the zero rows would make
-      // each store a partial-sector write that DRAM reads back to merge);
-      // force reads only the rows the bitmap names
-      masks[(size_t)r * n_total + i] = m;
-      if (m != 0u) hits |= 1 << r;
-      acc.add(part);
-    } else {
+      row_done(r, b[r] - base[r], len, bits, part);
+    }
+  } else if (MODE == MODE_DENSITY) {
+    // a CTA that spans too many columns or candidates to stage: rolled up, or
+    // the code of both forms would not stay in the instruction cache
+    const RowWindows w(S, pi, c, S->hl2);
+    const int zb = max(c.z - S->rz, 0);
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+      int rb, re;
+      w.range(S, start, c, r, rb, re);
+      int len = re - rb;
+      if (CWA_DCHECK_FAILED(len == 0 || (rb >= 0 && len > 0 && re <= n_total), status)) len = 0;
+      const int rbase = hits & kWindowMasks ? rb : row_valid(S, c, r) ? __ldg(start + row_id(S, c, r) + zb) : 0;
+      const float4* cand = pos + rb;
+      RowMask bits = 0u;
+      T part = (T)0;
+      if (len > 0) part = scan_row_prec<P, 2>([&](int o) { return __ldg(cand + o); }, len, pi, hit2, S->hs2, bits);
+      row_done(r, rb - rbase, len, bits, part);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      int len = e[r] - b[r];
+      if (CWA_DCHECK_FAILED(len == 0 || (b[r] >= 0 && len > 0 && e[r] <= n_total), status)) len = 0;
+      const int off0 = b[r] - base[r];
+      const float4* cand = pos + b[r];
       overflow |= off0 + len > kRowCodeMax;
       const uint32_t code0 = ((uint32_t)r << kRowCodeBits) + (uint32_t)off0;
-      if (len > 0) {
-        if (in_stage)
-          scan_row<false, T>([&](int o) { return cand[o]; }, len, code0, px, py, pz, hit2, hp, hp_end);
-        else
-          scan_row<false, T>([&](int o) { return __ldg(cand + o); }, len, code0, px, py, pz, hit2, hp, hp_end);
-      }
+      if (len > 0)
+        scan_row<false, T>([&](int o) { return __ldg(cand + o); }, len, code0, px, py, pz, hit2, hp, hp_end);
     }
   }
   if (MODE == MODE_LIST) {
