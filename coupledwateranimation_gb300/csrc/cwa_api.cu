@@ -64,8 +64,7 @@ struct cwa_sim {
   float4* XR = nullptr;        // positions at the last rebuild
   // force's gather records (x, y, z, p), (vx, vy, vz, 1/rho); 1/rho is in IR
   // (double) in FP64 mode
-  float4* XP = nullptr;
-  float4* VP = nullptr;
+  PairRec* PR = nullptr;
   double* IR = nullptr;
   int32_t* d_flag = nullptr;   // rebuild flag, raised by integrate / uploads
   unsigned long long* d_rebuilds = nullptr;
@@ -439,8 +438,7 @@ NbArgs nb_args(cwa_sim* s) {
   a.vlist = s->vlist;
   a.vcnt = s->vcnt;
   a.xref = s->XR;
-  a.xpair = s->XP;
-  a.vpair = s->VP;
+  a.pairs = s->PR;
   a.irho = s->IR;
   a.n_total = s->n_total;
   a.status = s->d_status;
@@ -955,8 +953,7 @@ cwa_status cwa_create(const cwa_sim_options* opt, const cwa_scene_desc* scenes, 
   ALLOC(s->nbm, N * kNbRows);
   ALLOC(s->nbr_cnt, N);
   ALLOC(s->KS, N);
-  ALLOC(s->XP, N);
-  ALLOC(s->VP, N);
+  ALLOC(s->PR, N);
   if (s->opt.precision == CWA_PREC_FP64) ALLOC(s->IR, N);
   ALLOC(s->d_flag, 1);
   ALLOC(s->d_rebuilds, 1);

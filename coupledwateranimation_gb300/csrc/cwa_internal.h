@@ -176,6 +176,11 @@ constexpr int kMaskBits = 64;
 constexpr int kWindowMasks = 1 << kNbRows;
 typedef uint64_t RowMask;  // one candidate row's hits, bit b = the candidate at the row's cell-based start + b
 constexpr int kMaxVerlet = 128;
+// A particle's gather record, one 32-byte sector.
+struct __align__(32) PairRec {
+  float4 xp;  // x, y, z, p
+  float4 vr;  // vx, vy, vz, 1/rho
+};
 struct NbArgs {
   const float4* pos;
   const float4* vel;
@@ -192,11 +197,9 @@ struct NbArgs {
   uint16_t* vlist;
   int32_t* vcnt;
   float4* xref;         // positions at the last rebuild (Verlet mode)
-  // (x, y, z, p) and (vx, vy, vz, 1/rho) of every particle, written by the
-  // density pass for force's neighbour gathers; FP64 has 1/rho in irho
-  // instead (null in the FP32 modes)
-  float4* xpair;
-  float4* vpair;
+  // written by the density pass for force's neighbour gathers; FP64 has 1/rho
+  // in irho instead (null in the FP32 modes)
+  PairRec* pairs;
   double* irho;
   int32_t n_total;
   int32_t* status;

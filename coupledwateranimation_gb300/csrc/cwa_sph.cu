@@ -219,17 +219,22 @@ __device__ __forceinline__ float2 eos(const SceneDev* S, float rho, float4 pi, c
   return make_float2(rho, p);
 }
 
-// Force's gather records of particle i: (x, y, z, p) and (vx, vy, vz, 1/rho),
-// so a pair costs two aligned 16-byte gathers; 1/rho uses force's recip.
-// FP64 keeps 1/rho in double beside them: one division a particle instead of
-// one a pair.
+// Force's gather record of particle i: (x, y, z, p) and (vx, vy, vz, 1/rho)
+// side by side, so a pair costs one aligned 32-byte gather; 1/rho uses force's
+// recip.  FP64 keeps 1/rho in double beside them: one division a particle
+// instead of one a pair.
+__device__ __forceinline__ void load_pair(const PairRec* __restrict__ rec, float4& x, float4& v) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(rec));
+}
+
 template <int P>
-__device__ __forceinline__ void write_pair_rec(float4* __restrict__ xp, float4* __restrict__ vp,
-                                               double* __restrict__ irho, const float4* __restrict__ vel, int i,
-                                               float4 pi, float2 rp) {
+__device__ __forceinline__ void write_pair_rec(PairRec* __restrict__ pairs, double* __restrict__ irho,
+                                               const float4* __restrict__ vel, int i, float4 pi, float2 rp) {
   const float4 v = __ldg(vel + i);
-  xp[i] = make_float4(pi.x, pi.y, pi.z, rp.y);
-  vp[i] = make_float4(v.x, v.y, v.z, P == CWA_PREC_FP64 ? 0.0f : recip(rp.x));
+  pairs[i].xp = make_float4(pi.x, pi.y, pi.z, rp.y);
+  pairs[i].vr = make_float4(v.x, v.y, v.z, P == CWA_PREC_FP64 ? 0.0f : recip(rp.x));
   if (P == CWA_PREC_FP64) irho[i] = recip((double)rp.x);
 }
 
@@ -616,8 +621,7 @@ __device__ __forceinline__ int scan_tile(
     const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const SceneDev* __restrict__ scenes,
     const float* __restrict__ wave, float2* __restrict__ rho_p, uint16_t* __restrict__ list,
     int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total,
-    int32_t* status, int32_t allow_stage, const float4* __restrict__ vel, float4* __restrict__ xpair,
-    float4* __restrict__ vpair, double* __restrict__ irho) {
+    int32_t* status, int32_t allow_stage, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho) {
   using T = Real<P>;
   constexpr int kCap = kMaxVerlet;  // the Verlet list build's codes per particle
   // The list build (rare: Verlet rebuilds only) reads candidates from global
@@ -765,7 +769,7 @@ __device__ __forceinline__ int scan_tile(
     const T rho_t = (P == CWA_PREC_FP64 ? (T)S->c_poly6_d : (T)S->c_poly6) * acc.get();
     const float2 rp = eos(S, (float)rho_t, pi, wave);
     rho_p[i] = rp;
-    write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
+    write_pair_rec<P>(pairs, irho, vel, i, pi, rp);
   }
   return used;
 }
@@ -782,8 +786,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
                  float2* __restrict__ rho_p, uint16_t* __restrict__ list, int32_t* __restrict__ list_cnt,
                  RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total, int32_t* status,
                  const int32_t* __restrict__ flag,
-                 int32_t allow_stage, const float4* __restrict__ vel, float4* __restrict__ xpair,
-                 float4* __restrict__ vpair, double* __restrict__ irho, const int32_t* __restrict__ order, int32_t* queue,
+                 int32_t allow_stage, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho, const int32_t* __restrict__ order, int32_t* queue,
                  int32_t n_tiles) {
   __shared__ ScanShared<MODE> sh;
   __shared__ int32_t s_next;
@@ -791,7 +794,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
   if (threadIdx.x == 0) mbar_init(&sh.bar, 1);
   if constexpr (!WQ || MODE != MODE_DENSITY) {
     scan_tile<P, MODE>(sh, tiles[blockIdx.x], 0u, pos, start, keys, scenes, wave, rho_p, list, list_cnt, masks,
-                       xref, n_total, status, allow_stage, vel, xpair, vpair, irho);
+                       xref, n_total, status, allow_stage, vel, pairs, irho);
     return;
   }
   uint32_t parity = 0u;
@@ -802,8 +805,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
     __syncthreads();  // s_next read by all before thread 0 may take the next number
     if (t >= n_tiles) break;
     const int used = scan_tile<P, MODE>(sh, tiles[__ldg(order + t)], parity, pos, start, keys, scenes, wave, rho_p,
-                                        list, list_cnt, masks, xref, n_total, status, allow_stage, vel, xpair,
-                                        vpair, irho);
+                                        list, list_cnt, masks, xref, n_total, status, allow_stage, vel, pairs, irho);
     if (__syncthreads_or(used & 2)) break;  // a staging wait timed out (status set): stop taking tiles
     if (used & 1) parity ^= 1u;
   }
@@ -821,8 +823,7 @@ __global__ void __launch_bounds__(kNbThreads, 8)
                const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                float2* __restrict__ rho_p, const uint16_t* __restrict__ vlist,
                const int32_t* __restrict__ vcnt, RowMask* __restrict__ nbm, int32_t* __restrict__ nbr_cnt,
-               int32_t n_total, const float4* __restrict__ vel, float4* __restrict__ xpair,
-               float4* __restrict__ vpair, double* __restrict__ irho) {
+               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho) {
   using T = Real<P>;
   __shared__ int32_t s_rb[9][kNbThreads];
   __shared__ RowMask s_m[kNbRows][kNbThreads];  // this step's row masks
@@ -904,7 +905,7 @@ __global__ void __launch_bounds__(kNbThreads, 8)
   const T rho_t = (P == CWA_PREC_FP64 ? (T)S->c_poly6_d : (T)S->c_poly6) * acc.get();
   const float2 rp = eos(S, (float)rho_t, pi, wave);
   rho_p[i] = rp;
-  write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
+  write_pair_rec<P>(pairs, irho, vel, i, pi, rp);
 }
 
 // The force a particle stores: pressure + viscosity sums (already scaled,
@@ -1023,8 +1024,7 @@ struct PairSums {
 // and the positions.
 struct PairArrays {
   const float4* __restrict__ pos;
-  const float4* __restrict__ xpair;
-  const float4* __restrict__ vpair;
+  const PairRec* __restrict__ pairs;
   const double* __restrict__ irho;
 };
 
@@ -1055,8 +1055,7 @@ __device__ __forceinline__ void add_hits(PairSums<P>& s, const PairArrays& a, in
     Real<P> ir[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      xj[u] = __ldg(a.xpair + js[u]);
-      vj[u] = __ldg(a.vpair + js[u]);
+      load_pair(a.pairs + js[u], xj[u], vj[u]);
       ir[u] = inv_rho<P>(a, vj[u], js[u]);
     }
 #pragma unroll
@@ -1122,17 +1121,17 @@ __device__ __forceinline__ void force_tile(
     const float4* __restrict__ pos, const float2* __restrict__ rho_p,
     const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const SceneDev* __restrict__ scenes,
     const float* __restrict__ wave, float4* __restrict__ force, const RowMask* __restrict__ nbm,
-    const int32_t* __restrict__ nbr_cnt, int32_t n_total, const float4* __restrict__ xpair,
-    const float4* __restrict__ vpair, const double* __restrict__ irho, int32_t* status) {
+    const int32_t* __restrict__ nbr_cnt, int32_t n_total, const PairRec* __restrict__ pairs, const double* __restrict__ irho, int32_t* status) {
   using T = Real<P>;
   const SceneDev* S = scenes + tl.scene;
   const int i = tl.begin + threadIdx.x;
   if (i >= tl.end) return;
   // the particle's own position and velocity come from its gather records
   // (the same floats, and lines its neighbours' gathers share)
-  const float4 pi = __ldg(xpair + i), vi = __ldg(vpair + i);
+  float4 pi, vi;
+  load_pair(pairs + i, pi, vi);
   const float2 rpi = __ldg(rho_p + i);
-  const PairArrays arrays{pos, xpair, vpair, irho};
+  const PairArrays arrays{pos, pairs, irho};
   PairSums<P> s;
   s.init(S, pi, vi, rpi.y);
   const int cnt = __ldg(nbr_cnt + i);
@@ -1179,7 +1178,8 @@ __device__ __forceinline__ void force_tile(
 #pragma unroll
       for (int u = 0; u < 8; ++u)
         if (js[u] >= 0 && !CWA_DCHECK_FAILED(js[u] < n_total, status)) {
-          const float4 xj = __ldg(xpair + js[u]), vj = __ldg(vpair + js[u]);
+          float4 xj, vj;
+          load_pair(pairs + js[u], xj, vj);
           s.pair(xj, vj, inv_rho<P>(arrays, vj, js[u]));
         }
       s.flush();
@@ -1208,7 +1208,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
             const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
             const SceneDev* __restrict__ scenes, const float* __restrict__ wave, float4* __restrict__ force,
             const RowMask* __restrict__ nbm, const int32_t* __restrict__ nbr_cnt, int32_t n_total,
-            const float4* __restrict__ xpair, const float4* __restrict__ vpair, const double* __restrict__ irho,
+            const PairRec* __restrict__ pairs, const double* __restrict__ irho,
             int32_t* status, const int32_t* __restrict__ order, int32_t* queue, int32_t n_tiles) {
   // the particle's nonzero row masks and the index of each mask's bit 0
   // (13.8 KB a CTA; 32-bit masks, 9.2 KB a CTA, measured slower: 209 against
@@ -1219,7 +1219,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
   __shared__ int32_t s_jb[kNbRows][kNbThreads];
   if constexpr (!WQ) {
     force_tile<P>(s_w, s_jb, tiles[blockIdx.x], pos, rho_p, start, keys, scenes, wave, force, nbm, nbr_cnt,
-                  n_total, xpair, vpair, irho, status);
+                  n_total, pairs, irho, status);
   } else {
     // work-queue form: resident CTAs take tile numbers from *queue
     __shared__ int32_t s_next[2];
@@ -1229,7 +1229,7 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
       const int t = s_next[it & 1];
       if (t >= n_tiles) break;
       force_tile<P>(s_w, s_jb, tiles[__ldg(order + t)], pos, rho_p, start, keys, scenes, wave, force, nbm,
-                    nbr_cnt, n_total, xpair, vpair, irho, status);
+                    nbr_cnt, n_total, pairs, irho, status);
     }
   }
 }
@@ -1296,8 +1296,7 @@ __global__ void __launch_bounds__(kNbThreads)
     k_rho_team(const float4* __restrict__ pos, const int32_t* __restrict__ start, const int32_t* __restrict__ keys,
                const Tile* __restrict__ tiles, const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                float2* __restrict__ rho_p, int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks,
-               int32_t n_total, const float4* __restrict__ vel, float4* __restrict__ xpair,
-               float4* __restrict__ vpair, double* __restrict__ irho, int32_t* status) {
+               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho, int32_t* status) {
   using R = Real<P>;
   const Tile tl = tiles[blockIdx.x / T];
   const int i = team_particle<T>(tl);
@@ -1353,7 +1352,7 @@ __global__ void __launch_bounds__(kNbThreads)
   const R rho_t = (P == CWA_PREC_FP64 ? (R)S->c_poly6_d : (R)S->c_poly6) * acc.get();
   const float2 rp = eos(S, (float)rho_t, pi, wave);
   rho_p[i] = rp;
-  write_pair_rec<P>(xpair, vpair, irho, vel, i, pi, rp);
+  write_pair_rec<P>(pairs, irho, vel, i, pi, rp);
 }
 
 // Force in the team form, for the cascaded sums only: their partials (8 hits,
@@ -1365,7 +1364,7 @@ __global__ void __launch_bounds__(kNbThreads, 6)
                  const int32_t* __restrict__ keys, const Tile* __restrict__ tiles,
                  const SceneDev* __restrict__ scenes, const float* __restrict__ wave, float4* __restrict__ force,
                  const RowMask* __restrict__ nbm, const int32_t* __restrict__ nbr_cnt, int32_t n_total,
-                 const float4* __restrict__ xpair, const float4* __restrict__ vpair, int32_t* status) {
+                 const PairRec* __restrict__ pairs, int32_t* status) {
   constexpr int P = CWA_PREC_COMPENSATED;
   __shared__ RowMask s_w[kNbRows][kNbThreads / T];
   __shared__ int32_t s_jb[kNbRows][kNbThreads / T];
@@ -1376,11 +1375,12 @@ __global__ void __launch_bounds__(kNbThreads, 6)
   const Team<T> team;
   const int tm = threadIdx.x / T;  // the team's column of the shared arrays
   const SceneDev* S = scenes + tl.scene;
-  const float4 pi = __ldg(xpair + i), vi = __ldg(vpair + i);
+  float4 pi, vi;
+  load_pair(pairs + i, pi, vi);
   const float2 rpi = __ldg(rho_p + i);
   const int cnt = __ldg(nbr_cnt + i);
   const CellCoord c = cell_of_key(S, __ldg(keys + i));
-  const PairArrays arrays{pos, xpair, vpair, nullptr};
+  const PairArrays arrays{pos, pairs, nullptr};
   PairSums<P> s;
   s.init(S, pi, vi, rpi.y);
   // Folds the lanes' partials in lane order: lane c keeps the sums of
@@ -1458,8 +1458,7 @@ __global__ void __launch_bounds__(kNbThreads, 6)
           float4 xj[4], vj[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            xj[u] = __ldg(xpair + js[h + u]);
-            vj[u] = __ldg(vpair + js[h + u]);
+            load_pair(pairs + js[h + u], xj[u], vj[u]);
           }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
@@ -1514,7 +1513,7 @@ void scan_launch_one(const NbArgs& a, uint16_t* list, int32_t* cnt, RowMask* mas
     grid = queue_grid(kern, a.tile_size, a.n_tiles);
   }
   kern<<<grid, a.tile_size, 0, st>>>(a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, list, cnt, masks,
-                                     xref, a.n_total, a.status, flag, a.stage, a.vel, a.xpair, a.vpair, a.irho, a.order,
+                                     xref, a.n_total, a.status, flag, a.stage, a.vel, a.pairs, a.irho, a.order,
                                      queue, a.n_tiles);
 }
 
@@ -1533,8 +1532,7 @@ template <int P>
 void dispatch_scan(bool list_mode, const NbArgs& a, cudaStream_t st) {
   if (!list_mode && a.team) {
     k_rho_team<P, kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
-        a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.xpair,
-        a.vpair, a.irho, a.status);
+        a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.pairs, a.irho, a.status);
     return;
   }
   if (list_mode)
@@ -1554,7 +1552,7 @@ void force_variant(const NbArgs& a, cudaStream_t st) {
     grid = queue_grid(kern, a.tile_size, a.n_tiles);
   }
   kern<<<grid, a.tile_size, 0, st>>>(a.pos, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm,
-                                     a.nbr_cnt, a.n_total, a.xpair, a.vpair, a.irho, a.status, a.order, queue,
+                                     a.nbr_cnt, a.n_total, a.pairs, a.irho, a.status, a.order, queue,
                                      a.n_tiles);
 }
 
@@ -1564,7 +1562,7 @@ void dispatch_force(const NbArgs& a, cudaStream_t st) {
     if (a.team) {
       k_force_team<kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
           a.pos, a.rho_p, a.start, a.keys, a.tiles, a.scenes, a.wave, a.force, a.nbm, a.nbr_cnt, a.n_total,
-          a.xpair, a.vpair, a.status);
+          a.pairs, a.status);
       return;
     }
   }
@@ -1598,7 +1596,7 @@ cudaError_t launch_rho_list(int precision, const NbArgs& a, cudaStream_t stream)
 #define CWA_RHO_LIST(P)                                                                                     \
   k_rho_list<P><<<a.n_tiles, a.tile_size, 0, stream>>>(a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave,  \
                                                        a.rho_p, a.vlist, a.vcnt, a.nbm, a.nbr_cnt, a.n_total, \
-                                                       a.vel, a.xpair, a.vpair, a.irho)
+                                                       a.vel, a.pairs, a.irho)
   switch (precision) {
     case CWA_PREC_FP32: CWA_RHO_LIST(CWA_PREC_FP32); break;
     case CWA_PREC_FP64: CWA_RHO_LIST(CWA_PREC_FP64); break;
