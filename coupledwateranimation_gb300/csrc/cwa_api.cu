@@ -318,20 +318,22 @@ void* host_alias(const void* host, size_t bytes) {
 }
 
 // One height field between the host and the device, on the sim's stream:
-// a kernel copy when the host side is page-locked and both sides are 16-byte
-// aligned, else cudaMemcpyAsync.
-cwa_status copy_field(cwa_sim* s, const float* src, float* dst, long cells, cudaMemcpyKind kind) {
+// a kernel copy when the host side is page-locked and all sides are 16-byte
+// aligned, else cudaMemcpyAsync.  dst2 (to the device): the copy again.
+cwa_status copy_field(cwa_sim* s, const float* src, float* dst, long cells, cudaMemcpyKind kind,
+                      float* dst2 = nullptr) {
   const bool to_dev = kind == cudaMemcpyHostToDevice;
   void* alias = host_alias(to_dev ? static_cast<const void*>(src) : static_cast<const void*>(dst),
                            (size_t)cells * sizeof(float));
   const float* dev_side = to_dev ? dst : src;
-  if (alias && !(reinterpret_cast<uintptr_t>(dev_side) & 15u)) {
+  if (alias && !((reinterpret_cast<uintptr_t>(dev_side) | reinterpret_cast<uintptr_t>(dst2)) & 15u)) {
     CWA_CUDA(launch_copy_f32(to_dev ? static_cast<const float*>(alias) : src,
-                             to_dev ? dst : static_cast<float*>(alias), cells, s->stream));
+                             to_dev ? dst : static_cast<float*>(alias), dst2, cells, s->stream));
     s->launches += 1;
     return CWA_OK;
   }
   CWA_CUDA(cudaMemcpyAsync(dst, src, (size_t)cells * sizeof(float), kind, s->stream));
+  if (dst2) CWA_CUDA(cudaMemcpyAsync(dst2, src, (size_t)cells * sizeof(float), kind, s->stream));
   return CWA_OK;
 }
 
@@ -1061,7 +1063,7 @@ cwa_status cwa_download_particles(cwa_sim* s, int32_t scene, cwa_particle* host,
   // page-locked destination then takes them in one coalesced kernel copy
   if (void* dst = host_alias(host, (size_t)n * sizeof(cwa_particle))) {
     CWA_CUDA(launch_copy_f32(reinterpret_cast<const float*>(s->staging), static_cast<float*>(dst),
-                             (long)n * (long)(sizeof(cwa_particle) / sizeof(float)), s->stream));
+                             nullptr, (long)n * (long)(sizeof(cwa_particle) / sizeof(float)), s->stream));
     s->launches += 1;
   } else {
     CWA_CUDA(cudaMemcpyAsync(host, s->staging, (size_t)n * sizeof(cwa_particle), cudaMemcpyDeviceToHost,
@@ -1078,8 +1080,9 @@ cwa_status cwa_upload_wave(cwa_sim* s, int32_t scene, const float* u_n, const fl
   if (nx != d.nx || nz != d.nz || !u_n) return arg_error("wave upload size must equal the scene's grid");
   const long cells = (long)nx * nz;
   const int w = s->wcur;
-  CWA_TRY(copy_field(s, u_n, s->U[w] + d.woff, cells, cudaMemcpyHostToDevice));
-  CWA_TRY(copy_field(s, u_nm1 ? u_nm1 : u_n, s->U[(w + 2) % 3] + d.woff, cells, cudaMemcpyHostToDevice));
+  float* const older = s->U[(w + 2) % 3] + d.woff;
+  CWA_TRY(copy_field(s, u_n, s->U[w] + d.woff, cells, cudaMemcpyHostToDevice, u_nm1 ? nullptr : older));
+  if (u_nm1) CWA_TRY(copy_field(s, u_nm1, older, cells, cudaMemcpyHostToDevice));
   CWA_CUDA(cudaStreamSynchronize(s->stream));
   return CWA_OK;
 }

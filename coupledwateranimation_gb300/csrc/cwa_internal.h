@@ -245,7 +245,7 @@ cudaError_t launch_unpack(const cwa_particle* aos, int32_t n, int32_t poff, floa
                           float4* force, float2* rho_p, float2* extra, int32_t* id, cudaStream_t stream);
 // n floats from src to dst, both 16-byte aligned (cudaErrorInvalidValue
 // otherwise); either may be the device address of page-locked host memory.
-cudaError_t launch_copy_f32(const float* src, float* dst, long n, cudaStream_t stream);
+cudaError_t launch_copy_f32(const float* src, float* dst, float* dst2, long n, cudaStream_t stream);
 cudaError_t launch_pack(cwa_particle* aos, int32_t n, int32_t poff, const float4* pos, const float4* vel,
                         const float4* force, const float2* rho_p, const float2* extra,
                         const int32_t* id, cudaStream_t stream);

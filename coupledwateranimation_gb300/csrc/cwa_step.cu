@@ -316,16 +316,17 @@ __global__ void __launch_bounds__(kLinkThreads)
   }
 }
 
-// Contiguous copy of n floats, both pointers 16-byte aligned, either side
-// device memory or page-locked host memory: 16-byte words, then the 0-3 floats
-// left.
+// Contiguous copy of n floats, pointers 16-byte aligned, either side device
+// memory or page-locked host memory: 16-byte words, then the 0-3 floats left.
+// With dst2 the copy is made twice from one read.
 template <int kDepth>
 __global__ void __launch_bounds__(kLinkThreads)
-    k_copy_f32(const float* __restrict__ src, float* __restrict__ dst, long n) {
+    k_copy_f32(const float* __restrict__ src, float* __restrict__ dst, float* __restrict__ dst2, long n) {
   const long n4 = n >> 2, stride = (long)gridDim.x * kLinkThreads;
   const long first = blockIdx.x * (long)kLinkThreads + threadIdx.x;
   const float4* s4 = reinterpret_cast<const float4*>(src);
   float4* d4 = reinterpret_cast<float4*>(dst);
+  float4* e4 = reinterpret_cast<float4*>(dst2);
   for (long t = first; t < n4; t += kDepth * stride) {
     float4 v[kDepth];
 #pragma unroll
@@ -333,9 +334,16 @@ __global__ void __launch_bounds__(kLinkThreads)
       if (t + u * stride < n4) v[u] = s4[t + u * stride];
 #pragma unroll
     for (int u = 0; u < kDepth; ++u)
-      if (t + u * stride < n4) d4[t + u * stride] = v[u];
+      if (t + u * stride < n4) {
+        d4[t + u * stride] = v[u];
+        if (dst2) e4[t + u * stride] = v[u];
+      }
   }
-  if (first < (n & 3)) dst[n4 * 4 + first] = src[n4 * 4 + first];
+  if (first < (n & 3)) {
+    const float v = src[n4 * 4 + first];
+    dst[n4 * 4 + first] = v;
+    if (dst2) dst2[n4 * 4 + first] = v;
+  }
 }
 
 inline unsigned link_grid(long words) {
@@ -473,12 +481,13 @@ cudaError_t launch_unpack(const cwa_particle* aos, int32_t n, int32_t poff, floa
   return cudaGetLastError();
 }
 
-cudaError_t launch_copy_f32(const float* src, float* dst, long n, cudaStream_t stream) {
+cudaError_t launch_copy_f32(const float* src, float* dst, float* dst2, long n, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(dst2)) & 15u)
+    return cudaErrorInvalidValue;
   const long words = (n >> 2) + 1;
   auto kern = words <= kLinkSmallWords ? k_copy_f32<1> : k_copy_f32<kLinkDepth>;
-  kern<<<link_grid(words), kLinkThreads, 0, stream>>>(src, dst, n);
+  kern<<<link_grid(words), kLinkThreads, 0, stream>>>(src, dst, dst2, n);
   return cudaGetLastError();
 }
 

@@ -32,3 +32,18 @@ def test_round_trip(lib, n):
         check(lib.cwa_download_wave(sim.handle, 0, ptr(v), None, n, 3), "download")
     assert np.array_equal(back.numpy(), rec.numpy())
     assert np.array_equal(v.numpy(), u.numpy())
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+@pytest.mark.parametrize("nx", [1, 7, 682, 683, 349526])
+def test_one_field_fills_both_levels(lib, nx, pinned):
+    import torch
+
+    sc = small_muller((3, 3, 3), 0.02, (nx, 3))
+    u = torch.from_numpy(np.random.default_rng(nx).uniform(-1, 1, (3, nx)).astype(np.float32))
+    u = u.pin_memory() if pinned else u
+    with Sim(sc.desc) as sim:
+        sim.upload_wave(0, u.numpy())
+        a, b = sim.download_wave(0)
+    assert np.array_equal(a, u.numpy())
+    assert np.array_equal(b, u.numpy())
