@@ -155,7 +155,8 @@ __device__ __forceinline__ void row_bases(const SceneDev* S, const int32_t* __re
 // An out-of-domain column is infinitely far, so one comparison rules out
 // either kind of row.  Nine windows a particle are a fifth of the density
 // pass's instructions, so each is kept short: one conversion that rounds down
-// a bound, no scaling around the square root.
+// a bound, no scaling around the square root (ten steps of 1M particles,
+// three sims interleaved, 3750 to 3585 us).
 struct RowWindows {
   float dxm, dxp, dym, dyp, zl, izc, zmax, rad2;
   __device__ __forceinline__ RowWindows(const SceneDev* S, float4 p, CellCoord c, float r2) {
@@ -220,8 +221,9 @@ __device__ __forceinline__ float2 eos(const SceneDev* S, float rho, float4 pi, c
 }
 
 // Force's gather record of particle i: (x, y, z, p) and (vx, vy, vz, 1/rho)
-// side by side, so a pair costs one aligned 32-byte gather; 1/rho uses force's
-// recip.  FP64 keeps 1/rho in double beside them: one division a particle
+// side by side, so a pair costs one aligned 32-byte gather (two of 16 bytes from
+// two arrays: ten steps of 1M particles, three sims interleaved, 3010 us for
+// 2868; 4.2M in FP32 5020 for 4740); 1/rho uses force's recip.  FP64 keeps 1/rho in double beside them: one division a particle
 // instead of one a pair.
 __device__ __forceinline__ void load_pair(const PairRec* __restrict__ rec, float4& x, float4& v) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -411,9 +413,9 @@ __device__ __forceinline__ T scan_row_bits(Load load, int len, T px, T py, T pz,
     const int n = min(len - c0, 32);
     uint32_t m = 0u, bit = 1u;
     // Unrolled by 2: a row holds ~12 candidates at C1 (z cells of h/4), so
-    // a deeper unroll spends its time in the remainder loop.  The candidate
-    // pass took 168 us unrolled by 4, 154 by 2, 165 by 1, 167 by 3 and 192
-    // by 8 at C1.
+    // a deeper unroll spends its time in the remainder loop.  With every CTA
+    // on this loop the pass took 168 us unrolled by 4, 154 by 2, 165 by 1, 167
+    // by 3 and 192 by 8 at C1; staged rows now go through scan_row_pairs.
 #pragma unroll U
     for (int o = 0; o < n; ++o) {
       const float4 pj = load(c0 + o);
@@ -540,7 +542,9 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
 // bit (zeros of an exact cancellation are +0 and the GPU's NaNs have none) and
 // goes into the mask with one funnel shift, and min(nq, 0) is what a hit adds
 // and nothing for a miss: 17 instructions a pair in place of 26, and the same
-// bits.
+// bits.  At 1M particles the pass went from 128M warp instructions and 129 us
+// to 109M and 122 (issue still bounds it, at 73%); unrolled by 1 or 4 three
+// interleaved sims' steps take 1.5% longer.
 __device__ __forceinline__ float scan_row_pairs(uint32_t stage, int o0, int len, float4 p, float h, RowMask& bits) {
   const F2 px = f2(p.x, p.x), py = f2(p.y, p.y), pz = f2(p.z, p.z), minus = f2(-1.0f, -1.0f);
   const float nh = -(h * h);
@@ -723,8 +727,13 @@ __device__ __forceinline__ int scan_tile(
       row_done(r, b[r] - base[r], len, bits, part);
     }
   } else if (MODE == MODE_DENSITY) {
-    // a CTA that spans too many columns or candidates to stage: rolled up, or
-    // the code of both forms would not stay in the instruction cache
+    // A CTA that spans too many columns or candidates to stage, rolled up.
+    // With both forms in each of the nine unrolled rows the pass took 123 us
+    // and not 117 at 1M particles, and ten steps of three interleaved sims
+    // 3585 us and not 3010: this way the kernel has 72 registers, and seven
+    // CTAs a SM where there were eight leave more of the SM's memory as L1 to
+    // the force CTAs of another sim (asking for the shared memory of eight
+    // brings 3690 us back).
     const RowWindows w(S, pi, c, S->hl2);
     const int zb = max(c.z - S->rz, 0);
 #pragma unroll 1
