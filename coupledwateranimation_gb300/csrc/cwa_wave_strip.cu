@@ -196,9 +196,10 @@ __device__ __forceinline__ void strip_fetch(const StripCtx& c, const float* row,
   cp_async16(dst, in ? row : field, in);
 }
 
-// The strip's columns of any row, from index at of the field on: the aligned words that cover it, 33 of them, as far as they start
-// inside the field (fields are padded to 128 bytes).  Columns outside the
-// domain hold whatever lies there, which no cell of the domain uses.
+// The strip's columns of any row, from index at of the field on: the aligned
+// words that cover it, 33 of them, as far as they start inside the field
+// (fields are padded to 128 bytes).  Columns outside the domain hold whatever
+// lies there, which no cell of the domain uses.
 __device__ __forceinline__ void strip_fetch_any(const StripCtx& c, const float* field, int at, bool row_in, int lane,
                                                 float* dst) {
   const int first = (at & ~(C - 1)) + C * lane, last = (at & ~(C - 1)) + kStripW, cells = c.W * c.H;
