@@ -182,7 +182,7 @@ __device__ bool collide(const PbdConst& c, const cwa_pbd_box& bi, const cwa_pbd_
 __global__ void __launch_bounds__(128)
     k_pbd_query(PbdConst c, cwa_pbd_box* __restrict__ boxes, const int32_t* __restrict__ cstart,
                 const int32_t* __restrict__ csorted, PbdPair* __restrict__ pairs, int32_t* __restrict__ npairs,
-                int32_t* __restrict__ rcount, int32_t* __restrict__ rlist, int32_t* status) {
+                int32_t* __restrict__ rcount, int64_t* __restrict__ rlist, int32_t* status) {
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= c.n) return;  // whole warps leave together
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(128)
       if (hit) {
         const int slot = t + __popc(hits & ((1u << lane) - 1u));
         if (slot < c.pcap) {
-          const int q = i * c.pcap + slot;
+          const int64_t q = (int64_t)i * c.pcap + slot;  // n x pcap goes up to 2^34
           pr.i = i;
           pr.j = j;
           pairs[q] = pr;
@@ -281,8 +281,8 @@ constexpr int kPostList = 64;
 __global__ void __launch_bounds__(kPostThreads)
     k_pbd_post(PbdConst c, cwa_pbd_box* __restrict__ boxes, const PbdPair* __restrict__ pairs,
                const int32_t* __restrict__ npairs, const int32_t* __restrict__ rcount,
-               const int32_t* __restrict__ rlist) {
-  __shared__ int32_t s_in[kPostThreads / kPostLanes][kPostList], s_out[kPostThreads / kPostLanes][kPostList];
+               const int64_t* __restrict__ rlist) {
+  __shared__ int64_t s_in[kPostThreads / kPostLanes][kPostList], s_out[kPostThreads / kPostLanes][kPostList];
   const int b = (blockIdx.x * kPostThreads + threadIdx.x) / kPostLanes;
   const int k = threadIdx.x % kPostLanes, g = threadIdx.x / kPostLanes;
   const unsigned team = 0xffu << ((threadIdx.x & 31) - k);
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kPostThreads)
     for (int s = k; s < nr; s += kPostLanes) s_in[g][s] = rlist[(size_t)b * c.pcap + s];
     __syncwarp(team);
     for (int s = k; s < nr; s += kPostLanes) {
-      const int q = s_in[g][s];
+      const int64_t q = s_in[g][s];
       int rank = 0;
       for (int m = 0; m < nr; ++m) rank += s_in[g][m] < q;
       s_out[g][rank] = q;
@@ -337,10 +337,10 @@ __global__ void __launch_bounds__(kPostThreads)
     for (int s = 0; s < nr; ++s) add(pairs[s_out[g][s]], false);
   } else if (nr <= c.pcap) {
     // entry by entry: the smallest one above the last
-    const int32_t* list = rlist + (size_t)b * c.pcap;
-    int last = -1;
+    const int64_t* list = rlist + (size_t)b * c.pcap;
+    int64_t last = -1;
     for (int s = 0; s < nr; ++s) {
-      int q = 0x7fffffff;
+      int64_t q = INT64_MAX;
       for (int m = k; m < nr; m += kPostLanes)
         if (list[m] > last) q = min(q, list[m]);
 #pragma unroll
@@ -395,7 +395,8 @@ struct cwa_pbd_sim {
   int32_t *ikey = nullptr, *islot = nullptr, *ccount = nullptr, *cstart = nullptr, *clist = nullptr,
           *csorted = nullptr;
   PbdPair* pairs = nullptr;
-  int32_t *npairs = nullptr, *rcount = nullptr, *rlist = nullptr;
+  int32_t *npairs = nullptr, *rcount = nullptr;
+  int64_t* rlist = nullptr;
   void* ws_cells = nullptr;
   ScanWorkspace scan_cells{};
   int32_t* d_status = nullptr;
@@ -523,7 +524,7 @@ cwa_status cwa_pbd_create(const cwa_pbd_params* p, int32_t device, cwa_pbd_sim**
   al((void**)&s->cstart, 4 * ((size_t)s->ncells + 1));
   al((void**)&s->pairs, sizeof(PbdPair) * slots);
   al((void**)&s->npairs, 4 * (size_t)k.n);
-  al((void**)&s->rlist, 4 * slots);
+  al((void**)&s->rlist, 8 * slots);
   al((void**)&s->rcount, 4 * (size_t)k.n);
   al(&s->ws_cells, scan_workspace_bytes(s->ncells + 1));
   al((void**)&s->d_status, 4);
