@@ -639,18 +639,17 @@ __device__ __forceinline__ int scan_tile(
   __syncthreads();
   const bool staged = kCanStage && allow_stage && sp.ncols > 0;
   if (staged && threadIdx.x < 32) {
-    // thread 0 arms the barrier with the stage's bytes, then lane s issues
-    // segment s's copy (at most 27 segments: one warp issues them all at once)
-    if (threadIdx.x == 0) mbar_expect_tx(&sh.bar, (uint32_t)sp.copied * 16u);
+    // lane s: segment s (at most 27: one warp issues all the copies at once)
+    const int s = threadIdx.x, len = s < 9 * sp.ncols ? sp.seg_len[s] : 0;
+    // an odd segment's last pair is filled up with a candidate out of reach,
+    // before thread 0 arms the barrier: its arrival releases the lanes' stores
+    // to the threads that wait on the barrier
+    const float far = __int_as_float(0x7f800000);
+    if (kPairs && (len & 1)) s_cand[sp.seg_off[s] + len] = make_float4(far, far, far, 0.0f);
     __syncwarp();
-    const int s = threadIdx.x;
-    if (s < 9 * sp.ncols) {
-      const int len = sp.seg_len[s];
-      // an odd segment's last pair is filled up with a candidate out of reach
-      const float far = __int_as_float(0x7f800000);
-      if (kPairs && (len & 1)) s_cand[sp.seg_off[s] + len] = make_float4(far, far, far, 0.0f);
-      if (len > 0) bulk_g2s(&s_cand[sp.seg_off[s]], pos + sp.seg_b[s], (uint32_t)len * 16u, &sh.bar);
-    }
+    if (s == 0) mbar_expect_tx(&sh.bar, (uint32_t)sp.copied * 16u);
+    __syncwarp();
+    if (len > 0) bulk_g2s(&s_cand[sp.seg_off[s]], pos + sp.seg_b[s], (uint32_t)len * 16u, &sh.bar);
   }
   bool ready = true;
   if (staged && !mbar_wait_bounded(&sh.bar, parity)) {
