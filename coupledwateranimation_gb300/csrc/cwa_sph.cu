@@ -157,17 +157,22 @@ __device__ __forceinline__ void row_bases(const SceneDev* S, const int32_t* __re
 // pass's instructions, so each is kept short: one conversion that rounds down
 // a bound, no scaling around the square root (ten steps of 1M particles,
 // three sims interleaved, 3750 to 3585 us).
+//
+// Every kernel forms the same window from the same position, bit for bit: the
+// masks of a dense spot count from the windows' starts, which the density pass
+// and force form in different kernels.  So each operation names its rounding
+// and none is left for the compiler to contract.
 struct RowWindows {
   float dxm, dxp, dym, dyp, zl, izc, zmax, rad2;
   __device__ __forceinline__ RowWindows(const SceneDev* S, float4 p, CellCoord c, float r2) {
-    const float x0f = S->lo[0] + (float)c.x * S->cell;
-    const float y0f = S->lo[1] + (float)c.y * S->cell;
+    const float x0f = __fmaf_rn((float)c.x, S->cell, S->lo[0]);
+    const float y0f = __fmaf_rn((float)c.y, S->cell, S->lo[1]);
     const float far = __int_as_float(0x7f800000);
-    dxm = c.x > 0 ? fmaxf(p.x - x0f, 0.0f) : far;
-    dxp = c.x + 1 < S->dims[0] ? fmaxf(x0f + S->cell - p.x, 0.0f) : far;
-    dym = c.y > 0 ? fmaxf(p.y - y0f, 0.0f) : far;
-    dyp = c.y + 1 < S->dims[1] ? fmaxf(y0f + S->cell - p.y, 0.0f) : far;
-    zl = p.z - S->lo[2];
+    dxm = c.x > 0 ? fmaxf(__fsub_rn(p.x, x0f), 0.0f) : far;
+    dxp = c.x + 1 < S->dims[0] ? fmaxf(__fsub_rn(__fadd_rn(x0f, S->cell), p.x), 0.0f) : far;
+    dym = c.y > 0 ? fmaxf(__fsub_rn(p.y, y0f), 0.0f) : far;
+    dyp = c.y + 1 < S->dims[1] ? fmaxf(__fsub_rn(__fadd_rn(y0f, S->cell), p.y), 0.0f) : far;
+    zl = __fsub_rn(p.z, S->lo[2]);
     izc = S->inv_cellz;
     zmax = (float)(S->dims[2] - 1);
     rad2 = r2;
