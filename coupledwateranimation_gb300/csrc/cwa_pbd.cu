@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(128)
           pr.j = j;
           pairs[q] = pr;
           const int s = atomicAdd(rcount + j, 1);
-          if (s < c.pcap) rlist[(size_t)j * c.pcap + s] = q;  // past pcap: the post pass searches the pairs
+          if (s < c.pcap) rlist[(size_t)j * c.pcap + s] = q;  // past pcap: long_partners finds them
         } else {
           atomicOr(status, kStatusBigCell);
         }
@@ -269,24 +269,148 @@ __global__ void __launch_bounds__(128)
 // fixed order, so a lane's chain is one addition a pair and the pairs' loads
 // are shared by the lanes and run ahead of the sums.  The box's partner list
 // is sorted first (each entry's rank is the number of smaller ones), in shared
-// memory up to kPostList entries; longer lists, rare, are taken smallest entry
-// first, and one past its pcap slots is replaced by a search of all pairs in
-// slot order.  One thread a box took 22 us at 4096 boxes, this
+// memory; boxes of more than kPostList partners, or more than their list holds,
+// go to long_partners.  One thread a box took 22 us at 4096 boxes, this
 // form 11 us, and the list replaces a counting sort of all pair slots (a key
 // pass, a scan and two passes over n pcap slots, 19 us).
 constexpr int kPostLanes = 8;
 constexpr int kPostThreads = 128;
+constexpr int kPostTeams = kPostThreads / kPostLanes;
 constexpr int kPostList = 64;
+constexpr int kPostWindow = 1 << 17;  // boxes a window of long_partners, a bit each
 
-__global__ void __launch_bounds__(kPostThreads)
+struct PostShared {
+  union {
+    struct {
+      int64_t in[kPostTeams][kPostList], out[kPostTeams][kPostList];
+    };
+    uint32_t bits[kPostWindow / 32];
+  };
+  float val[kPostThreads][6];  // long_partners: the values of up to 128 pairs
+  int32_t low[kPostThreads];   // and the pairs' lower boxes
+  int32_t warp[kPostThreads / 32], next, is_long[kPostTeams];
+};
+
+// Adds the partner pairs of box b, whose team is `mine`, in slot order, that is
+// by lower box (a box has one pair at most with another), with the whole block.
+// The partners share a cell with b, so they are found among the members of b's
+// cells: each marks its bit in a window of box numbers if it has a pair with b,
+// and the bits name the pairs in order, 128 at a time.  The members are walked
+// once a window.  What it costs is a few loads a member, shared by 128 threads;
+// the query's one warp has walked the same members.  With one large box of
+// the highest index over n - 1 small ones, 64 slots a box, a step takes 493 us
+// at 4096 boxes and 5,076 at 20,000; with the box's team alone walking every
+// lower box's pairs it took 3,382 and 43,375, and with partners from a
+// counting sort of all pair slots 2,861 and 19,440.
+__device__ __forceinline__ float long_partners(const PbdConst& c, int b, const cwa_pbd_box* boxes,
+                                            const PbdPair* __restrict__ pairs, const int32_t* __restrict__ npairs,
+                                            const int32_t* __restrict__ cstart,
+                                            const int32_t* __restrict__ csorted, PostShared& sh, bool mine,
+                                            float sum) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int lo[3], hi[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = cell_c(c, fs(boxes[b].x[a], boxes[b].hw[a]), a);
+    hi[a] = cell_c(c, fa(boxes[b].x[a], boxes[b].hw[a]), a);
+  }
+  const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1, rows = (hi[0] - lo[0] + 1) * ny;
+  auto slot_of = [&](int i) {  // box i's pair with b, or -1
+    const int m = npairs[i];
+    const PbdPair* p = pairs + (size_t)i * c.pcap;
+    for (int t = 0; t < m; t += 4) {  // four loads in flight
+      int j[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) j[u] = t + u < m ? p[t + u].j : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j[u] == b) return t + u;
+    }
+    return -1;
+  };
+  const volatile uint32_t* const bits = sh.bits;  // other warps set bits while a warp looks
+  int w0 = 0;  // the window's first box
+  while (w0 < b) {
+    const int per = min((b - w0 - 1) / (32 * kPostThreads) + 1, kPostWindow / 32 / kPostThreads);  // words a thread
+    for (int w = tid; w < per * kPostThreads; w += kPostThreads) sh.bits[w] = 0u;
+    if (tid == 0) sh.next = b;
+    __syncthreads();
+    int next = b;  // the first member past the window
+    for (int row = warp; row < rows; row += kPostThreads / 32) {
+      const int x = row / ny, cell0 = cell_id(c, lo[0] + x, lo[1] + row - x * ny, lo[2]);
+      const int e = cstart[cell0 + nz];
+      for (int m = cstart[cell0] + lane; m < e; m += 32) {
+        const int i = csorted[m], at = i - w0;
+        if (i >= b || at < 0) continue;
+        if (at >= kPostWindow) {
+          next = min(next, i);
+        } else if (!(bits[at >> 5] >> (at & 31) & 1u) && slot_of(i) >= 0) {
+          atomicOr(&sh.bits[at >> 5], 1u << (at & 31));
+        }
+      }
+    }
+    next = __reduce_min_sync(0xffffffffu, next);
+    if (lane == 0) atomicMin(&sh.next, next);
+    __syncthreads();
+    // each thread's words, and the number of bits before them
+    int own = 0;
+    for (int w = 0; w < per; ++w) own += __popc(sh.bits[tid * per + w]);
+    int incl = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += y;
+    }
+    if (lane == 31) sh.warp[warp] = incl;
+    __syncthreads();
+    int first = incl - own, total = 0;
+    for (int w = 0; w < kPostThreads / 32; ++w) {
+      if (w < warp) first += sh.warp[w];
+      total += sh.warp[w];
+    }
+    for (int r0 = 0; r0 < total; r0 += kPostThreads) {
+      if (first < r0 + kPostThreads && first + own > r0) {
+        int r = first - r0;
+        for (int w = 0; w < per; ++w)
+          for (uint32_t m = sh.bits[tid * per + w]; m; m &= m - 1u, ++r)
+            if (r >= 0 && r < kPostThreads) sh.low[r] = w0 + 32 * (tid * per + w) + __ffs((int)m) - 1;
+      }
+      __syncthreads();
+      const int n = min(total - r0, kPostThreads);
+      if (tid < n) {
+        const int i = sh.low[tid];
+        const PbdPair& pr = pairs[(size_t)i * c.pcap + slot_of(i)];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          sh.val[tid][a] = fm(pr.wj, pr.disp[a]);
+          sh.val[tid][a + 3] = fm(pr.wj, pr.frict[a]);
+        }
+      }
+      __syncthreads();
+      if (mine) {
+        const int k = tid % kPostLanes;
+#pragma unroll 8
+        for (int r = 0; r < n; ++r) sum = fa(sum, k < 6 ? sh.val[r][min(k, 5)] : 1.0f);
+      }
+      __syncthreads();
+    }
+    w0 = sh.next;
+    __syncthreads();
+  }
+  return sum;
+}
+
+__global__ void __launch_bounds__(kPostThreads, 8)
     k_pbd_post(PbdConst c, cwa_pbd_box* __restrict__ boxes, const PbdPair* __restrict__ pairs,
                const int32_t* __restrict__ npairs, const int32_t* __restrict__ rcount,
-               const int64_t* __restrict__ rlist) {
-  __shared__ int64_t s_in[kPostThreads / kPostLanes][kPostList], s_out[kPostThreads / kPostLanes][kPostList];
-  const int b = (blockIdx.x * kPostThreads + threadIdx.x) / kPostLanes;
+               const int64_t* __restrict__ rlist, const int32_t* __restrict__ cstart,
+               const int32_t* __restrict__ csorted) {
+  __shared__ PostShared sh;
   const int k = threadIdx.x % kPostLanes, g = threadIdx.x / kPostLanes;
+  const int b0 = blockIdx.x * kPostTeams;
+  const bool live = b0 + g < c.n;
+  const int b = live ? b0 + g : c.n - 1;  // teams past the end compute the last box and store nothing
   const unsigned team = 0xffu << ((threadIdx.x & 31) - k);
-  if (b >= c.n) return;  // whole teams leave together
   const cwa_pbd_box o = boxes[b];
   float dpn[3] = {0.0f, 0.0f, 0.0f}, dpt[3] = {0.0f, 0.0f, 0.0f}, nn = 0.0f;
   // collisions with the extents (:230-259), on every lane
@@ -323,37 +447,24 @@ __global__ void __launch_bounds__(kPostThreads)
 #pragma unroll 4
   for (int t = 0; t < no; ++t) add(mine[t], true);  // b is the lower box
   const int nr = rcount[b];  // b is the higher box
+  const bool is_long = live && (nr > kPostList || nr > c.pcap);
   if (nr <= kPostList && nr <= c.pcap) {
-    for (int s = k; s < nr; s += kPostLanes) s_in[g][s] = rlist[(size_t)b * c.pcap + s];
+    for (int s = k; s < nr; s += kPostLanes) sh.in[g][s] = rlist[(size_t)b * c.pcap + s];
     __syncwarp(team);
     for (int s = k; s < nr; s += kPostLanes) {
-      const int64_t q = s_in[g][s];
+      const int64_t q = sh.in[g][s];
       int rank = 0;
-      for (int m = 0; m < nr; ++m) rank += s_in[g][m] < q;
-      s_out[g][rank] = q;
+      for (int m = 0; m < nr; ++m) rank += sh.in[g][m] < q;
+      sh.out[g][rank] = q;
     }
     __syncwarp(team);
 #pragma unroll 4
-    for (int s = 0; s < nr; ++s) add(pairs[s_out[g][s]], false);
-  } else if (nr <= c.pcap) {
-    // entry by entry: the smallest one above the last
-    const int64_t* list = rlist + (size_t)b * c.pcap;
-    int64_t last = -1;
-    for (int s = 0; s < nr; ++s) {
-      int64_t q = INT64_MAX;
-      for (int m = k; m < nr; m += kPostLanes)
-        if (list[m] > last) q = min(q, list[m]);
-#pragma unroll
-      for (int x = 1; x < kPostLanes; x <<= 1) q = min(q, __shfl_xor_sync(team, q, x, kPostLanes));
-      add(pairs[q], false);
-      last = q;
-    }
-  } else {
-    for (int i = 0; i < b; ++i)
-      for (int t = 0; t < npairs[i]; ++t) {
-        const PbdPair& pr = pairs[(size_t)i * c.pcap + t];
-        if (pr.j == b) add(pr, false);
-      }
+    for (int s = 0; s < nr; ++s) add(pairs[sh.out[g][s]], false);
+  }
+  if (k == 0) sh.is_long[g] = is_long;
+  if (__syncthreads_or(is_long)) {
+    for (int q = 0; q < kPostTeams; ++q)
+      if (sh.is_long[q]) sum = long_partners(c, b0 + q, boxes, pairs, npairs, cstart, csorted, sh, g == q, sum);
   }
   nn = __shfl_sync(team, sum, 6, kPostLanes);
   const int a = k < 3 ? k : 0;
@@ -367,7 +478,7 @@ __global__ void __launch_bounds__(kPostThreads)
   const float moved = fs(ox, p);
   const bool awake = len3(__shfl_sync(team, moved, 0, kPostLanes), __shfl_sync(team, moved, 1, kPostLanes),
                           __shfl_sync(team, moved, 2, kPostLanes)) > c.sleep;
-  if (k < 3) {
+  if (live && k < 3) {
     cwa_pbd_box& w = boxes[b];
     w.v[a] = fd(fs(pe, ox), c.dt);
     w.dp_n[a] = dn;
@@ -455,7 +566,7 @@ cwa_status enqueue_substep(cwa_pbd_sim* s) {
   k_pbd_query<<<nb(32l * c.n), kB, 0, st>>>(c, s->boxes, s->cstart, s->csorted, s->pairs, s->npairs, s->rcount,
                                             s->rlist, s->d_status);
   k_pbd_post<<<(unsigned)(((long)c.n * kPostLanes + kPostThreads - 1) / kPostThreads), kPostThreads, 0, st>>>(
-      c, s->boxes, s->pairs, s->npairs, s->rcount, s->rlist);
+      c, s->boxes, s->pairs, s->npairs, s->rcount, s->rlist, s->cstart, s->csorted);
   PBD_CUDA(cudaGetLastError());
   return CWA_OK;
 }
