@@ -794,7 +794,6 @@ cwa_status read_status2(cwa2d_sim* s) {
   if (v == 0) return CWA_OK;
   CWA2_CUDA(cudaMemsetAsync(s->d_status, 0, 4, s->stream));
   CWA2_CUDA(cudaStreamSynchronize(s->stream));
-  if (v & kStatusTimeout) return err2("a bounded device wait (scan look-back) timed out", CWA_ERR_TIMEOUT);
   if (v & kStatusNonFinite) return err2("non-finite particle position", CWA_ERR_NONFINITE);
   return err2("a grid cell held more than 1024 particles; its insert order fell back to arrival order",
               CWA_ERR_CAPACITY);

@@ -208,7 +208,15 @@ __global__ void __launch_bounds__(kScanBlock)
 // tiles before it to its own local scan (k_tile_scan).  The input is read
 // twice (4.8 MB at the 1M-particle grid, from L2 the second time) but no
 // tile waits on another, where the look-back chain of k_scan kept each CTA
-// resident ~12 us for a ~5 us job.
+// resident ~12 us for a ~5 us job.  Adding up the totals before it is work
+// that grows with the square of the tiles, so above kSumTiles tiles a launch
+// between the two scans the totals (k_scan_sums).  Point grid builds of
+// 100,000 points, us without / with that launch / with k_scan:
+//   2^23 cells (1,025 tiles)    41.9 /   41.7 /   65
+//   2^24                        70.1 /   67.9 /   98
+//   2^25                         134 /    125 /  182
+//   2^27                         513 /    406 /  629
+//   2^30                      14,068 /  2,957 / 4,782
 template <bool kVec>
 __device__ __forceinline__ void load_tile_items(const int32_t* in, int32_t n_in, long base, int (&v)[kScanItems]) {
   if (kVec) {
@@ -256,10 +264,53 @@ __global__ void __launch_bounds__(kScanBlock)
   }
 }
 
+constexpr int kSumTiles = 1024;
+constexpr int kSumThreads = 1024;
+constexpr int kSumItems = 8;
+
+// The tiles' totals scanned in place, by one CTA.
+__global__ void __launch_bounds__(kSumThreads) k_scan_sums(int32_t* sums, int32_t n_tiles, const int32_t* flag) {
+  chain_enter();
+  if (flag && __ldg(flag) == 0) return;
+  __shared__ int s_warp[kSumThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int base = 0; base < n_tiles; base += kSumThreads * kSumItems) {
+    int v[kSumItems], t = 0;
+    const int first = base + (int)threadIdx.x * kSumItems;
+#pragma unroll
+    for (int k = 0; k < kSumItems; ++k) {
+      const int x = first + k < n_tiles ? sums[first + k] : 0;
+      v[k] = t;
+      t += x;
+    }
+    int incl = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int excl = before + incl - t, total = 0;
+#pragma unroll
+    for (int w = 0; w < kSumThreads / 32; ++w) {
+      if (w < warp) excl += s_warp[w];
+      total += s_warp[w];
+    }
+    before += total;
+#pragma unroll
+    for (int k = 0; k < kSumItems; ++k)
+      if (first + k < n_tiles) sums[first + k] = excl + v[k];
+    __syncthreads();
+  }
+}
+
+// scanned: sums holds the totals' scan.
 template <bool kZero, bool kVec>
 __global__ void __launch_bounds__(kScanBlock)
     k_tile_scan(int32_t* in, int32_t* out, int32_t n_in, int32_t n_out, const int32_t* __restrict__ sums,
-                const int32_t* flag) {
+                bool scanned, const int32_t* flag) {
   chain_enter();
   if (flag && __ldg(flag) == 0) return;
   __shared__ int s_warp[kScanBlock / 32];
@@ -268,9 +319,11 @@ __global__ void __launch_bounds__(kScanBlock)
   const int tile = blockIdx.x;
   if (warp == 0) {  // the totals of the tiles before this one
     int p = 0;
-    for (int t = lane; t < tile; t += 32) p += sums[t];
-    p = warp_sum(p);
-    if (lane == 0) s_prefix = p;
+    if (!scanned) {
+      for (int t = lane; t < tile; t += 32) p += sums[t];
+      p = warp_sum(p);
+    }
+    if (lane == 0) s_prefix = scanned ? sums[tile] : p;
   }
   const long base = (long)tile * kScanTile + (long)threadIdx.x * kScanItems;
   int v[kScanItems];
@@ -510,18 +563,23 @@ cudaError_t scan_launch_two_pass(int32_t* in, int32_t* out, int32_t n_in, int32_
       e = launch_chained(k_tile_sum<false>, grid, block, 0, stream, in, n_in, sums, flag);
     if (e != cudaSuccess) return e;
   }
+  const bool scanned = ws.n_tiles > kSumTiles;
+  if (scanned) {
+    e = launch_chained(k_scan_sums, dim3(1), dim3(kSumThreads), 0, stream, sums, ws.n_tiles, flag);
+    if (e != cudaSuccess) return e;
+  }
   if (zero_input) {
     if (vec)
-      e = launch_chained(k_tile_scan<true, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
+      e = launch_chained(k_tile_scan<true, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
     else
-      e = launch_chained(k_tile_scan<true, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
+      e = launch_chained(k_tile_scan<true, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
   } else {
     if (vec)
-      e = launch_chained(k_tile_scan<false, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
+      e = launch_chained(k_tile_scan<false, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
     else
-      e = launch_chained(k_tile_scan<false, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, flag);
+      e = launch_chained(k_tile_scan<false, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
   }
-  if (launches) *launches += ws.n_tiles > 1 ? 2 : 1;
+  if (launches) *launches += 1 + (ws.n_tiles > 1) + scanned;
   return e;
 }
 

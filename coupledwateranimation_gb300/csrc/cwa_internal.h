@@ -126,7 +126,8 @@ cudaError_t scan_launch(const int32_t* in, int32_t* out, int32_t n_in, int32_t n
                         const int32_t* flag = nullptr);
 
 // The same scan as two chained kernels (tile totals, then every tile's
-// scan plus the totals before it); uses the workspace's tile-state area for
+// scan plus the totals before it; for very many tiles a third between them
+// scans the totals); uses the workspace's tile-state area for
 // the totals, needs no zeroing and has no wait that can time out.
 cudaError_t scan_launch_two_pass(int32_t* in, int32_t* out, int32_t n_in, int32_t n_out, bool zero_input,
                                  const ScanWorkspace& ws, cudaStream_t stream, int64_t* launches,

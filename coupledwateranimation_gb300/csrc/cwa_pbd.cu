@@ -578,7 +578,6 @@ cwa_status read_pbd_status(cwa_pbd_sim* s) {
   if (v == 0) return CWA_OK;
   PBD_CUDA(cudaMemsetAsync(s->d_status, 0, 4, s->stream));
   PBD_CUDA(cudaStreamSynchronize(s->stream));
-  if (v & kStatusTimeout) return perr("a bounded device wait (scan look-back) timed out", CWA_ERR_TIMEOUT);
   if (v & kStatusNonFinite) return perr("non-finite box position", CWA_ERR_NONFINITE);
   return perr("a box overlapped more cells, or had more contacts, than its slots hold", CWA_ERR_CAPACITY);
 }

@@ -391,9 +391,9 @@ cwa_status cwa_grid_build(const float* d_pos4, int32_t n, const float lo[3], flo
                           int32_t* d_cell_of, void* d_workspace, size_t workspace_bytes,
                           void* stream);
 /* Waits for `stream`, then reports the last cwa_grid_build on this
- * workspace with these sizes: CWA_OK, CWA_ERR_NONFINITE (a NaN/Inf point),
- * CWA_ERR_TIMEOUT (a scan look-back gave up) or CWA_ERR_CAPACITY (a cell
- * above 1024 points: that cell's order fell back to arrival order). */
+ * workspace with these sizes: CWA_OK, CWA_ERR_NONFINITE (a NaN/Inf point)
+ * or CWA_ERR_CAPACITY (a cell above 1024 points: that cell's order fell back
+ * to arrival order). */
 cwa_status cwa_grid_status(int32_t n, int32_t n_cells, const void* d_workspace, void* stream);
 
 /* ---- headless rendering (the reference's display(), Main.cpp:326-474) ----
