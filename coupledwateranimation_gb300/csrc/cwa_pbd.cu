@@ -507,7 +507,7 @@ struct cwa_pbd_sim {
           *csorted = nullptr;
   PbdPair* pairs = nullptr;
   int32_t *npairs = nullptr, *rcount = nullptr;
-  int64_t* rlist = nullptr;
+  int64_t* rlist = nullptr;  // behind the pairs, in their allocation
   void* ws_cells = nullptr;
   ScanWorkspace scan_cells{};
   int32_t* d_status = nullptr;
@@ -547,8 +547,7 @@ void free_pbd(cwa_pbd_sim* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->graph) cudaGraphExecDestroy(s->graph);
   free_items(s);
-  void* ps[] = {s->boxes,  s->ccount, s->cstart,   s->pairs,   s->npairs,
-                s->rcount, s->rlist,  s->ws_cells, s->d_status};
+  void* ps[] = {s->boxes, s->ccount, s->cstart, s->pairs, s->npairs, s->rcount, s->ws_cells, s->d_status};
   for (void* p : ps) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
@@ -632,9 +631,9 @@ cwa_status cwa_pbd_create(const cwa_pbd_params* p, int32_t device, cwa_pbd_sim**
   al((void**)&s->boxes, sizeof(cwa_pbd_box) * k.n);
   al((void**)&s->ccount, 4 * (size_t)s->ncells);
   al((void**)&s->cstart, 4 * ((size_t)s->ncells + 1));
-  al((void**)&s->pairs, sizeof(PbdPair) * slots);
+  al((void**)&s->pairs, (sizeof(PbdPair) + sizeof(int64_t)) * slots);
+  if (e == cudaSuccess) s->rlist = reinterpret_cast<int64_t*>(s->pairs + slots);
   al((void**)&s->npairs, 4 * (size_t)k.n);
-  al((void**)&s->rlist, 8 * slots);
   al((void**)&s->rcount, 4 * (size_t)k.n);
   al(&s->ws_cells, scan_workspace_bytes(s->ncells + 1));
   al((void**)&s->d_status, 4);
