@@ -68,10 +68,10 @@ class SimOptions(C.Structure):
                 ("nb_queue", C.c_int32), ("reserved", C.c_int32 * 2)]
 
 
-# CWA_WAVE_BLOCK_*: register strips (the default), then box rows x steps per launch; R = box column in registers,
-# P = 256-wide box with column pairs in registers, S = persistent register
-# form with the next box prefetched
-WAVE_BLOCKS = ("strip", "64x4", "64x8", "R32x4", "R64x4", "R64x8", "P32x4", "S32x4")
+# CWA_WAVE_BLOCK_*: register strips (the default), then box rows x steps per
+# launch; R = box column in registers, P = 256-wide box with column pairs in
+# registers, S = persistent register form with the next box prefetched
+WAVE_BLOCKS = ("strip", "64x4", "64x8", "R32x4", "R64x4", "R64x8", "P32x4", "S32x4", "32x4")
 
 
 class WaveTuneReport(C.Structure):

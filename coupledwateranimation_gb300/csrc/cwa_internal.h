@@ -260,10 +260,11 @@ cudaError_t launch_totals(const float4* pos, const float4* vel, int32_t poff, in
 // ---- temporally blocked wave advance (cwa_wave_tma.cu) ----
 // Block variants from 1 on (box 128 x 64 / K 4 and K 8 with the column walk in
 // shared memory; 128 x 32 / K 4, 128 x 64 / K 4 and K 8 with it in registers;
-// a 256 x 32 / K 4 box with column pairs in registers; and a persistent
-// register-column form that prefetches each CTA's next 128 x 32 box): K wave
-// steps per launch, equal to the halo width.
-constexpr int kWaveVariants = 8;
+// a 256 x 32 / K 4 box with column pairs in registers; a persistent
+// register-column form that prefetches each CTA's next 128 x 32 box; and the
+// 128 x 32 / K 4 box with the walk in shared memory): K wave steps per launch,
+// equal to the halo width.
+constexpr int kWaveVariants = 9;
 int wave_variant_steps(int variant);
 
 // One block tile: patch (bx, by) of a scene's field; tma = rows load by TMA.

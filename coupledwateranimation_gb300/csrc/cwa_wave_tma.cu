@@ -41,9 +41,9 @@ constexpr int kWaveTmaThreads = kBoxW;  // one thread per box column
 // The block variants the tuner chooses from: box height and steps per launch
 // (= halo).  Output patch (128 - 2K) x (BOX_H - 2K).  Entry 0 stands for the
 // strips, which are no box.
-constexpr int kVarBoxW[kWaveVariants] = {128, 128, 128, 128, 128, 128, 256, 128};
-constexpr int kVarBoxH[kWaveVariants] = {32, 64, 64, 32, 64, 64, 32, 32};
-constexpr int kVarK[kWaveVariants] = {4, 4, 8, 4, 4, 8, 4, 4};
+constexpr int kVarBoxW[kWaveVariants] = {128, 128, 128, 128, 128, 128, 256, 128, 128};
+constexpr int kVarBoxH[kWaveVariants] = {32, 64, 64, 32, 64, 64, 32, 32, 32};
+constexpr int kVarK[kWaveVariants] = {4, 4, 8, 4, 4, 8, 4, 4, 4};
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
@@ -716,6 +716,7 @@ cudaError_t launch_wave_block(const WaveBlockArgs& a, int32_t n_tiles, int varia
     case 4: return launch_variant<64, 4, kReg>(a, n_tiles, stream);
     case 5: return launch_variant<64, 8, kReg>(a, n_tiles, stream);
     case 6: return launch_variant<32, 4, kPair>(a, n_tiles, stream);
+    case 8: return launch_variant<32, 4, kShared>(a, n_tiles, stream);
     default: return cudaErrorInvalidValue;  // variant 0 is the strips (cwa_wave_strip.cu)
   }
 }

@@ -138,12 +138,12 @@ typedef struct cwa_sim_options {
 
 /* Wave advance variants.  STRIP (the default): warps march up strips of 128
  * columns held in registers, 2 to 8 steps per launch.  The others: box of
- * 128 x H cells (P: 256 x H) advanced K steps per launch in shared memory; the R and P variants hold each
- * thread's box column (P: column pair) in registers and exchange only the
- * east / west neighbours through shared memory. */
+ * 128 x H cells (P: 256 x H) advanced K steps per launch in shared memory;
+ * the R and P variants hold each thread's box column (P: column pair) in
+ * registers and exchange only the east / west neighbours through shared
+ * memory. */
 enum {
   CWA_WAVE_BLOCK_STRIP = 0,
-  CWA_WAVE_BLOCK_32x4 = 0,  /* the default's earlier name */
   CWA_WAVE_BLOCK_64x4 = 1,  /* H 64, K 4 */
   CWA_WAVE_BLOCK_64x8 = 2,  /* H 64, K 8 */
   CWA_WAVE_BLOCK_R32x4 = 3, /* registers, H 32, K 4 */
@@ -152,7 +152,10 @@ enum {
   CWA_WAVE_BLOCK_P32x4 = 6, /* registers, 256 x 32 box, two columns a thread, K 4 */
   CWA_WAVE_BLOCK_S32x4 = 7, /* registers, H 32, K 4, persistent CTAs that prefetch
                                their next box while walking the current one */
-  CWA_WAVE_BLOCK_COUNT = 8
+  CWA_WAVE_BLOCK_32x4 = 8,  /* H 32, K 4; up to 8% faster than the strips on
+                               fields of 1 to 2M cells where several sims
+                               share the GPU, 10 to 20% slower alone */
+  CWA_WAVE_BLOCK_COUNT = 9
 };
 
 /* Borrowed device pointers of one scene, all in the current sorted order.
