@@ -406,20 +406,28 @@ void drop_graphs(cwa_sim* s) {
 // Whether the density and force passes run with four lanes a particle.
 // Small sims leave the GPU idle and each pass lasts as long as its longest
 // thread, so they share a particle among lanes; the team forms issue more
-// instructions in all, so larger sims keep one thread.  Measured step times
-// (us; one sim, and per step with three sims' steps interleaved; one thread /
-// four lanes, dam break, z cells of h):
-//    4,096 particles: 37 / 28 and 13.9 / 11.0
-//    8,000:           47 / 30 and 18.3 / 12.8
-//   18,816:           49 / 36 and 21.1 / 18.4
-//   32,768:           43 / 47 and 28.2 / 25.7
-//   64,000:           60 / 71 and 37.2 / 43.3
-// (Two lanes lie between: 38 and 17.2 at 18,816, but 5% slower than one thread
-// at 32,768 when uploads interleave.)  The work-queue option keeps its own
-// form.
+// instructions in all, so larger sims keep one thread.  Step times of a dam
+// break (us; one sim, and per step with three sims' steps interleaved), for
+// one thread / two lanes / four:
+//   compensated, z cells of h (FP32 and z cells of h / 4 are alike)
+//    4,096 particles: 36.8 / 32.2 / 27.3 and 13.4 / 12.0 / 10.8
+//    8,000:           48.5 / 35.0 / 31.0 and 18.2 / 13.4 / 12.6
+//   18,816:           52.0 / 39.1 / 37.2 and 20.1 / 16.5 / 18.4
+//   24,389:           54.2 / 41.6 / 37.1 and 21.4 / 17.6 / 17.9
+//   32,768:           42.5 / 43.3 / 46.9 and 18.7 / 21.2 / 26.0
+//   FP64 (the density pass alone has the form)
+//    4,096:            102 / 94 / 87 and 35.1 / 33.3 / 35.9
+//    8,000:            109 / 97 / 93 and 49.2 / 48.0 / 50.3
+//   18,816:            116 / 109 / 114 and 72.5 / 79.0 / 89.1
+//   24,389:            158 / 153 / 161 and 89.7 / 99.5 / 116
+// Two lanes are the better number only where sims interleave near the limit.
+// Any option of the one-thread forms that is set (stage, CTA size, launch
+// bounds, work queue) asks for those forms.
 bool use_team(const cwa_sim* s) {
   constexpr int32_t kTeamMaxParticles = 24 * 1024;
-  return !s->opt.nb_queue && s->n_total <= kTeamMaxParticles;
+  const cwa_sim_options& o = s->opt;
+  const bool chosen = o.nb_queue || o.nb_threads || o.nb_stage || o.nb_scan_minb || o.nb_force_minb;
+  return !chosen && s->n_total <= kTeamMaxParticles;
 }
 
 NbArgs nb_args(cwa_sim* s) {
@@ -1512,22 +1520,29 @@ cwa_status cwa_autotune(cwa_sim* s, int32_t trial_steps, cwa_tune_report* out) {
   if (err == cudaSuccess) err = cudaEventCreate(&e1);
   const int stages[2] = {0, -1}, scans[3] = {4, 6, 8}, forces[2] = {8, 9}, ctas[2] = {128, 64};
   constexpr int kCombos = 2 * 3 * 2 * 2;
+  // A small sim's default is none of the combinations (they are one-thread
+  // forms): its entry options are a trial of their own, the last.
+  const bool entry_team = use_team(s);
+  const int trials = kCombos + entry_team;
   // Two rounds, the second in reverse order; each combination keeps its
   // faster round, which damps clock and neighbour-load noise.
-  float best_of[kCombos];
+  float best_of[kCombos + 1];
   for (float& v : best_of) v = 1e30f;
   for (int round = 0; round < 2 && err == cudaSuccess; ++round)
-    for (int q = 0; q < kCombos && err == cudaSuccess; ++q) {
-      const int idx = round == 0 ? q : kCombos - 1 - q;
+    for (int q = 0; q < trials && err == cudaSuccess; ++q) {
+      const int idx = round == 0 ? q : trials - 1 - q;
       const int a = idx / 12, b = (idx / 4) % 3, c = (idx / 2) % 2, d = idx % 2;
       cwa_sim_options o = entry;
-      o.nb_stage = stages[a];
-      o.nb_scan_minb = scans[b];
-      o.nb_force_minb = forces[c];
-      o.nb_threads = ctas[d];
+      if (idx < kCombos) {
+        o.nb_stage = stages[a];
+        o.nb_scan_minb = scans[b];
+        o.nb_force_minb = forces[c];
+        o.nb_threads = ctas[d];
+      }
       s->opt = o;
-      if (s->ptile != ctas[d]) {
-        cwa_status st = set_particle_tiles(s, ctas[d]);
+      const int32_t ptile = idx < kCombos ? ctas[d] : entry_ptile;
+      if (s->ptile != ptile) {
+        cwa_status st = set_particle_tiles(s, ptile);
         if (st != CWA_OK) {
           err = cudaErrorMemoryAllocation;
           break;
@@ -1552,7 +1567,8 @@ cwa_status cwa_autotune(cwa_sim* s, int32_t trial_steps, cwa_tune_report* out) {
       if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e0, e1);
       ms /= (float)trial_steps;
       best_of[idx] = std::min(best_of[idx], ms);
-      if (round == 1) {
+      if (idx == kCombos) rep.entry_ms = best_of[idx];
+      if (round == 1 && idx < kCombos) {
         ms = best_of[idx];
         if (rep.n_tried < CWA_TUNE_MAX_TRIED) {
           rep.tried[rep.n_tried] = o;
@@ -1560,7 +1576,7 @@ cwa_status cwa_autotune(cwa_sim* s, int32_t trial_steps, cwa_tune_report* out) {
         }
         rep.n_tried++;
         // the entry options, with 0 read as each knob's default
-        if ((o.nb_stage < 0) == (entry.nb_stage < 0) &&
+        if (!entry_team && (o.nb_stage < 0) == (entry.nb_stage < 0) &&
             o.nb_scan_minb == (entry.nb_scan_minb ? entry.nb_scan_minb : 4) &&
             o.nb_force_minb == (entry.nb_force_minb ? entry.nb_force_minb : 9) &&
             o.nb_threads == (entry.nb_threads ? entry.nb_threads : 128))

@@ -116,7 +116,12 @@ typedef struct cwa_sim_options {
   int32_t device;          /* CUDA device ordinal                             */
   int32_t precision;       /* CWA_PREC_*                                      */
   int32_t use_graph;       /* capture cwa_step into CUDA graphs               */
-  int32_t nb_threads;      /* threads per CTA of the neighbour passes; 0=auto */
+  int32_t nb_threads;      /* threads per CTA of the neighbour passes; 0=auto.
+                              A sim of up to 24,576 particles that sets none
+                              of this, nb_stage, nb_scan_minb, nb_force_minb
+                              and nb_queue runs the density pass (and, with
+                              CWA_PREC_COMPENSATED, force) with four lanes a
+                              particle instead of one.  Same results.       */
   int32_t nb_stage;        /* density pass stages candidate rows in shared
                               memory: 0/1 = on (default), -1 = off         */
   float verlet_skin;       /* 0: sort and scan neighbours every step.  > 0:
@@ -319,10 +324,11 @@ cwa_status cwa_get_launch_count(cwa_sim* sim, int64_t* launches);
 /* ---- autotuner ------------------------------------------------------------
  * Tries the neighbour-pass kernel variants on the sim's current state
  * (candidate staging on/off, launch-bound variants of the density scan and
- * force, 128- or 64-particle CTAs), each from the same snapshot for
- * trial_steps timed steps, keeps the fastest (unless it beats the options at
- * entry by less than 1.5%, which is within the trials' noise) and restores
- * the state.  It allocates a snapshot of the state while it runs. */
+ * force, 128- or 64-particle CTAs; a small sim's several-lanes form stands
+ * for its options at entry), each from the same snapshot for trial_steps
+ * timed steps, keeps the fastest (unless it beats the options at entry by
+ * less than 1.5%, which is within the trials' noise) and restores the
+ * state.  It allocates a snapshot of the state while it runs. */
 #define CWA_TUNE_MAX_TRIED 32
 typedef struct cwa_tune_report {
   cwa_sim_options best;
