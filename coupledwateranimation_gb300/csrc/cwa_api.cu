@@ -421,13 +421,15 @@ void drop_graphs(cwa_sim* s) {
 //   18,816:            116 / 109 / 114 and 72.5 / 79.0 / 89.1
 //   24,389:            158 / 153 / 161 and 89.7 / 99.5 / 116
 // Two lanes are the better number only where sims interleave near the limit.
+// In FP64 the pass is bound by the FP64 pipe, which four lanes load no less,
+// so it gains only while one thread a particle does not fill the SMs.
 // Any option of the one-thread forms that is set (stage, CTA size, launch
 // bounds, work queue) asks for those forms.
 bool use_team(const cwa_sim* s) {
-  constexpr int32_t kTeamMaxParticles = 24 * 1024;
+  constexpr int32_t kTeamMaxParticles = 24 * 1024, kTeamMaxFp64 = 8 * 1024;
   const cwa_sim_options& o = s->opt;
   const bool chosen = o.nb_queue || o.nb_threads || o.nb_stage || o.nb_scan_minb || o.nb_force_minb;
-  return !chosen && s->n_total <= kTeamMaxParticles;
+  return !chosen && s->n_total <= (o.precision == CWA_PREC_FP64 ? kTeamMaxFp64 : kTeamMaxParticles);
 }
 
 NbArgs nb_args(cwa_sim* s) {

@@ -117,9 +117,10 @@ typedef struct cwa_sim_options {
   int32_t precision;       /* CWA_PREC_*                                      */
   int32_t use_graph;       /* capture cwa_step into CUDA graphs               */
   int32_t nb_threads;      /* threads per CTA of the neighbour passes; 0=auto.
-                              A sim of up to 24,576 particles that sets none
-                              of this, nb_stage, nb_scan_minb, nb_force_minb
-                              and nb_queue runs the density pass (and, with
+                              A sim of up to 24,576 particles (8,192 with
+                              CWA_PREC_FP64) that sets none of this, nb_stage,
+                              nb_scan_minb, nb_force_minb and nb_queue runs
+                              the density pass (and, with
                               CWA_PREC_COMPENSATED, force) with four lanes a
                               particle instead of one.  Same results.       */
   int32_t nb_stage;        /* density pass stages candidate rows in shared

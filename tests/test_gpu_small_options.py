@@ -71,7 +71,7 @@ def test_options_reach_their_kernels(lib, prec, zsub):
         assert np.array_equal(g, got[0]), kw
 
 
-@pytest.mark.parametrize("prec,n", [(PREC_FP32, 24576), (PREC_COMPENSATED, 24576), (PREC_FP64, 24576)])
+@pytest.mark.parametrize("prec,n", [(PREC_FP32, 24576), (PREC_COMPENSATED, 24576), (PREC_FP64, 8192)])
 def test_limit_of_the_several_lanes_forms(lib, prec, n):
     sc = small_muller((30, 30, 30), 0.02, (16, 16), seed=2)
     for count in (n, n + 1):
