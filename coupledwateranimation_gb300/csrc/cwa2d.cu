@@ -141,8 +141,18 @@ __global__ void k2_hash(Sph2dConst c, const float4* __restrict__ pos, int32_t* _
 // 17.9 us a substep at 4096 particles, this and the rank 8.8 (cold caches).
 // (The whole build in one CTA with shared-memory counters took 20: one SM's
 // issue slots.)
+// Every CTA scans every counter, so the work grows with particles x counters;
+// a launch saved is worth 1 to 2 us.  Frames of two substeps, one sim / three
+// interleaved, us, with the scan and the insert as two launches and as this one
+// (particles, cells):
+//    4,096, 16^2  56.9 / 22.7 and 54.5 / 22.0    4,096, 32^2  50.0 / 20.0 and 49.2 / 19.5
+//    4,096, 45^2  54.4 / 22.1 and 54.7 / 24.2    4,096, 63^2  56.2 / 23.3 and 60.7 / 25.9
+//   16,384, 32^2   115 / 64.1 and  113 / 64.2   32,768, 32^2   221 /  155 and  220 /  153
+// and grid passes alone at 131,072, 32^2 52.8 and 54.4, at 1,048,576 247 and 252.
 constexpr int kScanThreads = 256;
-constexpr int kScanMaxCells = 4096;
+constexpr int kScanMaxCells = 1280;
+constexpr long kScanMaxWork = 1l << 25;
+inline bool one_launch_grid(int n, int nb) { return nb <= kScanMaxCells && (long)n * nb <= kScanMaxWork; }
 
 __global__ void __launch_bounds__(kScanThreads)
     k2_scan_insert(int n, int nb, const int32_t* __restrict__ count, const int32_t* __restrict__ key,
@@ -689,7 +699,7 @@ cwa_status pass_grid(cwa2d_sim* s) {
     CWA2_CUDA(cudaGetLastError());
   }
   s->counts_pending = false;  // the rank pass clears them
-  if (nb <= kScanMaxCells) {
+  if (one_launch_grid(c.n, nb)) {
     k2_scan_insert<<<(unsigned)((c.n + kScanThreads - 1) / kScanThreads), kScanThreads, 0, s->stream>>>(
         c.n, nb, s->count, s->key, s->slot, s->start, s->list);
     CWA2_CUDA(cudaGetLastError());
