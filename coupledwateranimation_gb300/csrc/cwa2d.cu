@@ -573,12 +573,20 @@ __global__ void k1_wave_iter(Sph2dConst c, const float4* __restrict__ cur, const
   wave1_cell(c, cur, prev, out, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// All wave substeps of a frame in one CTA, for fields of at most kWaveCells
-// cells: a substep is a barrier instead of a launch (3.7 us each: two of a
-// frame's launches with the shallow-water kind, ten with Wave1D's ten substeps;
-// one launch of this form takes 5.6 us with the shallow-water kind).  w[0..2]: the buffers in the order of
-// the phase w0 = the newest field's index.
-constexpr int kWaveCells = 4096;
+// All wave substeps of a frame in one CTA, where they would be two launches or
+// more: a substep's passes are a barrier apart instead of a launch.  Beyond a
+// cell a thread the one CTA falls behind.  Frames of wave substeps only, us,
+// launches and this form:
+//   cells                       128         512        1,024       2,048       4,096
+//   shallow water, 1 substep    8.3  6.2    8.2  6.2   6.2  6.2    6.2  8.2    6.8 10.3
+//   shallow water, 4           14.4  8.2   16.4  8.2  20.5 14.4   20.5 18.5   20.5 28.7
+//   Wave1D, 1                   4.1  5.0    4.1  4.1   4.1  6.2    4.1  6.2    4.1  8.2
+//   Wave1D, 10                 16.1  6.5   17.1 10.3  17.8 12.3   18.5 23.1   19.2 37.7
+// w[0..2]: the buffers in the order of the phase; w0: the newest field's index.
+constexpr int kWaveCells = 1024;
+inline bool one_cta_wave(int kind, int cells, int substeps) {
+  return cells <= kWaveCells && substeps >= (kind == CWA2D_WAVE_1D ? 2 : 1);
+}
 struct WaveBuffers {
   float4* w[3];
 };
@@ -777,7 +785,7 @@ cwa_status enqueue_frame(cwa2d_sim* s) {
     if (st == CWA_OK) st = pass_sph(s, false);
     if (st != CWA_OK) return st;
   }
-  if (s->k.wave_n <= kWaveCells && s->prm.wave_substeps > 0) {
+  if (one_cta_wave(s->k.wave_kind, s->k.wave_n, s->prm.wave_substeps)) {
     k2_wave_frame<<<1, 1024, 0, s->stream>>>(s->k, WaveBuffers{{s->W[0], s->W[1], s->W[2]}}, s->wcur,
                                              s->prm.wave_substeps);
     CWA2_CUDA(cudaGetLastError());

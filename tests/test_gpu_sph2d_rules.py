@@ -1,12 +1,13 @@
 """The 2D family on either side of the sizes where its grid changes its kernels,
-its cells and its particles times cells, against the CPU restatement."""
+its cells and its particles times cells, against the CPU restatement; and
+where a frame's wave substeps change theirs, against single passes."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
 from test_gpu_sph2d_grid import TOL, _params, _rel_inf, _state
-from coupledwateranimation_gb300.sim2d import Sim2D
+from coupledwateranimation_gb300.sim2d import Sim2D, defaults2d
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +34,23 @@ def test_grid_rule(lib, orc, n, cells):
     want_f = orc.force_2d(p, dens, wave, grid_from=state)
     for k in range(2):
         assert _rel_inf(forc["acc"][:, k], want_f["acc"][:, k]) <= TOL
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("substeps", [1, 2, 5])
+@pytest.mark.parametrize("cells", [3, 1023, 1024, 1025, 2049])
+def test_wave_rule(lib, cells, substeps, kind):
+    p = defaults2d(kind)
+    p.n_particles, p.init_columns = 64, 8
+    p.sph_substeps, p.wave_substeps, p.wave_cells = 0, substeps, cells
+    names = ("wave_iterate",) if kind else ("wave_predict", "wave_correct")
+    with Sim2D(p) as a, Sim2D(p) as b:
+        a.splash()
+        b.splash()
+        a.step(3)
+        for _ in range(3 * substeps):
+            for name in names:
+                b.run_pass(name)
+        assert np.array_equal(a.download_wave().view(np.uint32), b.download_wave().view(np.uint32))
+        if kind:
+            assert np.array_equal(a.download_wave_prev().view(np.uint32), b.download_wave_prev().view(np.uint32))
