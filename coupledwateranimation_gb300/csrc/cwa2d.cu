@@ -120,17 +120,21 @@ __device__ __forceinline__ int bucket_of(const Sph2dConst& c, float4 p) {
                 : c.ncx * c.ncy;
 }
 
-__device__ __forceinline__ void hash_particle(const Sph2dConst& c, int i, float4 p, int32_t* __restrict__ key,
-                                              int32_t* __restrict__ slot, int32_t* __restrict__ count) {
+// One lane of a warp alone.
+__device__ __forceinline__ void hash_one(const Sph2dConst& c, int i, float4 p, int32_t* __restrict__ key,
+                                         int32_t* __restrict__ slot, int32_t* __restrict__ count) {
   const int k = bucket_of(c, p);
   key[i] = k;
-  slot[i] = count_slot(count, k);
+  slot[i] = atomicAdd(count + k, 1);
 }
 
 __global__ void k2_hash(Sph2dConst c, const float4* __restrict__ pos, int32_t* __restrict__ key,
                         int32_t* __restrict__ slot, int32_t* __restrict__ count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < c.n) hash_particle(c, i, pos[i], key, slot, count);
+  if (i >= c.n) return;
+  const int k = bucket_of(c, pos[i]);
+  key[i] = k;
+  slot[i] = count_slot(count, k);
 }
 
 // Small grids: every CTA scans all the counters itself (its own copy of the
@@ -362,7 +366,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
       pout[ix] = p;
       vout[ix] = v;
       aout[ix] = a;
-      hash_particle(c, ix, p, key, slot, count);
+      hash_one(c, ix, p, key, slot, count);
     }
     return;
   }
@@ -433,7 +437,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   pout[ix] = p;
   vout[ix] = v;
   aout[ix] = a;
-  hash_particle(c, ix, p, key, slot, count);
+  hash_one(c, ix, p, key, slot, count);
 }
 
 // InitParticle / init_grid (:308-333).

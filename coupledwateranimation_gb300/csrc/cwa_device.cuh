@@ -49,30 +49,43 @@ __device__ __forceinline__ bool finite3(float4 p) {
   return isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
 }
 
-// Warp-aggregated count: a run of neighbouring lanes with the same key shares
-// one atomicAdd; each lane's slot is its arrival rank within the cell.  Runs
-// catch what matters (particles near cell order; equal keys of scattered
-// points are rare in a warp) for a shuffle and a ballot.  The point grid's
-// build of 1,000,003 scattered points / of the same points sorted, 125 a cell:
-// 59 / 50 us with all equal keys grouped by match.any, 48 / 85 with one atomic
-// a point, 41 / 45 with runs (the last with one memset less, ~2 us).
+// Warp-aggregated count: the lanes of a warp with the same key share one
+// atomicAdd; each lane's slot is its arrival rank within the cell.  The lanes
+// are grouped by five bits of a multiplicative hash of the key, a ballot a bit;
+// of a group the lanes that hold its first lane's key go together, of the rest
+// those that hold the rest's first key, any others (three keys of one hash
+// among 32 lanes) each alone.
+// Point grid builds of 1,000,003 points, us, with the atomics of runs of equal
+// neighbours joined / of all equal keys by match.any / by this:
+//   scattered over 8,192 cells              58 /  66 /  58
+//   sorted, all in one cell                 46 /  46 /  46
+//   two cells in turn                      360 /  46 /  46
+//   every other one in one cell, the rest scattered over 400,000
+//                                          355 /  54 /  52
+// match.any takes a step for each distinct key of the warp; runs leave equal
+// keys with others between them to the memory system, one by one.
 __device__ __forceinline__ int count_slot(int32_t* count, int key) {
   const unsigned int active = __activemask();
   const int lane = threadIdx.x & 31;
-  const int prev = __shfl_up_sync(active, key, 1);
-  const bool first = lane == 0 || !((active >> (lane - 1)) & 1u) || prev != key;
-  const unsigned int firsts = __ballot_sync(active, first);
-  // the run: from the nearest first at or below this lane to the lane before
-  // the next first or the next inactive lane
-  const int begin = 31 - __clz(firsts & (0xffffffffu >> (31 - lane)));
-  int base = 0;
-  if (first) {
-    const unsigned int stop = (firsts | ~active) & ~(0xffffffffu >> (31 - lane));  // lanes above this one
-    const int end = stop ? __ffs(stop) - 1 : 32;
-    base = atomicAdd(count + key, end - lane);
+  const unsigned int hash = ((unsigned int)key * 0x9e3779b1u) >> 27;
+  unsigned int peers = active;
+#pragma unroll
+  for (int b = 0; b < 5; ++b) {
+    const bool bit = (hash >> b) & 1u;
+    const unsigned int set = __ballot_sync(active, bit);
+    peers &= bit ? set : ~set;
   }
-  base = __shfl_sync(active, base, begin);
-  return base + lane - begin;
+#pragma unroll
+  for (int round = 0; round < 2; ++round) {
+    const bool same = __shfl_sync(active, key, __ffs((int)peers) - 1) == key;
+    const unsigned int all = __ballot_sync(active, same);
+    peers &= same ? all : round == 0 ? ~all : 1u << lane;
+  }
+  const int leader = __ffs((int)peers) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(count + key, __popc(peers));
+  base = __shfl_sync(active, base, leader);
+  return base + __popc(peers & ((1u << lane) - 1u));
 }
 
 // texture(wave_tex, uv) with GL_LINEAR / GL_CLAMP_TO_EDGE on an R32F image
