@@ -579,7 +579,7 @@ cwa_status prepare_wave_strips(cwa_sim* s) {
   int sms = 0;
   CWA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
   std::vector<WaveStrip> strips;
-  for (int k = 2; k <= kWaveStripMaxSteps; ++k) {
+  for (int k = kWaveStripMinSteps; k <= kWaveStripMaxSteps; ++k) {
     s->strip_off[k] = (int32_t)strips.size();
     wave_strips(s->sd, k, sms, &strips);
   }
@@ -624,7 +624,9 @@ cwa_status prepare_wave_boxes(cwa_sim* s) {
 
 // n wave passes: a single pass first when deposits are pending (it applies
 // and clears them), launches of K steps of the sim's wave_block variant (the
-// default takes 2 to 8 steps a launch), single passes for the remainder.
+// default takes 4 to 8 steps a launch), single passes for the remainder and
+// for calls of fewer than 4 steps: those need no memory, keep the buffers'
+// pointers and with them the captured step graphs.
 // A launch writes u^(n+K) into the free slot and u^(n+K-1) into the spare; the
 // slots are then renamed so U[wcur] / U[(wcur+2)%3] hold them, which is the
 // state K single passes leave (up to the rotation of wcur).
@@ -651,8 +653,9 @@ cwa_status run_wave_advance(cwa_sim* s, int32_t n) {
   if (v == 0) {
     // as few launches as 8 steps each allow, of as equal a number of steps as
     // possible: a remainder run as 4 + 1 took a third of 773 x 1021's 29 steps
-    if (n - done >= 2) CWA_TRY(prepare_wave_strips(s));
-    for (int32_t left = n - done; left >= 2; left = n - done) {
+    // (from 4 steps on that is 4 to 8 a launch)
+    if (n - done >= kWaveStripMinSteps) CWA_TRY(prepare_wave_strips(s));
+    for (int32_t left = n - done; left >= kWaveStripMinSteps; left = n - done) {
       const int32_t launches = (left + kWaveStripMaxSteps - 1) / kWaveStripMaxSteps;
       const int32_t K = (left + launches - 1) / launches;
       WaveStripArgs a;

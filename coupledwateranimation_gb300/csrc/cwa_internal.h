@@ -308,7 +308,8 @@ struct WaveStripArgs {
   float neg_zero = -0.0f;  // see mul2
 };
 constexpr int kWaveStripMinRows = 16;
-constexpr int kWaveStripMaxSteps = 8;  // a launch takes 2 .. 8 steps
+constexpr int kWaveStripMinSteps = 4;  // a launch takes 4 .. 8 steps
+constexpr int kWaveStripMaxSteps = 8;
 // The strips of every scene for `steps` steps a launch.
 void wave_strips(const std::vector<SceneDev>& scenes, int steps, int sms, std::vector<WaveStrip>* out);
 cudaError_t launch_wave_strips(const WaveStripArgs& a, int32_t n_strips, int steps, cudaStream_t stream);

@@ -412,8 +412,6 @@ cudaError_t launch_wave_strips(const WaveStripArgs& a, int32_t n_strips, int ste
     else                                                                      \
       k_wave_strip<K, false><<<grid, kStripThreads, 0, stream>>>(a, n_strips); \
     break
-    CWA_STRIP(2);
-    CWA_STRIP(3);
     CWA_STRIP(4);
     CWA_STRIP(5);
     CWA_STRIP(6);

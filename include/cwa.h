@@ -143,7 +143,7 @@ typedef struct cwa_sim_options {
 } cwa_sim_options;
 
 /* Wave advance variants.  STRIP (the default): warps march up strips of 128
- * columns held in registers, 2 to 8 steps per launch.  The others: box of
+ * columns held in registers, 4 to 8 steps per launch.  The others: box of
  * 128 x H cells (P: 256 x H) advanced K steps per launch in shared memory;
  * the R and P variants hold each thread's box column (P: column pair) in
  * registers and exchange only the east / west neighbours through shared
@@ -282,8 +282,10 @@ cwa_status cwa_pass_wave(cwa_sim* sim);
  * StencilImage2DTripleBuffered.cpp:22-31 and wave_comp.glsl EvolveWave
  * :171-206, one dispatch per step).  Bit-identical to n_steps calls of
  * cwa_pass_wave; deposits pending from an integrate pass land in the first
- * step.  Steps run several per launch (the sim's wave_block option), so device pointers of the wave buffers may
- * change: re-read cwa_get_device_view after it.  Asynchronous. */
+ * step.  Steps run several per launch (the sim's wave_block option), so
+ * device pointers of the wave buffers may change: re-read
+ * cwa_get_device_view after it.  Fewer than 4 steps run as single passes and
+ * allocate nothing.  Asynchronous. */
 cwa_status cwa_wave_advance(cwa_sim* sim, int32_t n_steps);
 /* Wait for the sim's stream; report a device-side status (timeout, NaN). */
 cwa_status cwa_synchronize(cwa_sim* sim);
