@@ -734,8 +734,8 @@ cwa_status pass_sph(cwa2d_sim* s, bool density) {
   if (density) {
     if (!s->psort_fresh)  // a second density pass on the same grid
       k2_order<<<blocks(n), kBlock, 0, s->stream>>>(n, s->P[a], s->sorted, s->psort);
-    k2_density<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b], s->A[b],
-                                                              s->start, s->psort, s->inv, s->rec, s->pr,
+    k2_density<<<grid, 32 * kWarpsPerBlock, 0, s->stream>>>(s->k, s->P[a], s->V[a], s->A[a], s->P[b], s->V[b],
+                                                              s->A[b], s->start, s->psort, s->inv, s->rec, s->pr,
                                                               s->W[s->wcur]);
   } else {
     if (!s->rec_fresh)  // a force pass straight after the grid's

@@ -570,14 +570,18 @@ cudaError_t scan_launch_two_pass(int32_t* in, int32_t* out, int32_t n_in, int32_
   }
   if (zero_input) {
     if (vec)
-      e = launch_chained(k_tile_scan<true, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
+      e = launch_chained(k_tile_scan<true, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned,
+                         flag);
     else
-      e = launch_chained(k_tile_scan<true, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
+      e = launch_chained(k_tile_scan<true, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned,
+                         flag);
   } else {
     if (vec)
-      e = launch_chained(k_tile_scan<false, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
+      e = launch_chained(k_tile_scan<false, true>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned,
+                         flag);
     else
-      e = launch_chained(k_tile_scan<false, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned, flag);
+      e = launch_chained(k_tile_scan<false, false>, grid, block, 0, stream, in, out, n_in, n_out, sums, scanned,
+                         flag);
   }
   if (launches) *launches += 1 + (ws.n_tiles > 1) + scanned;
   return e;

@@ -228,8 +228,9 @@ __device__ __forceinline__ float2 eos(const SceneDev* S, float rho, float4 pi, c
 // Force's gather record of particle i: (x, y, z, p) and (vx, vy, vz, 1/rho)
 // side by side, so a pair costs one aligned 32-byte gather (two of 16 bytes from
 // two arrays: ten steps of 1M particles, three sims interleaved, 3010 us for
-// 2868; 4.2M in FP32 5020 for 4740); 1/rho uses force's recip.  FP64 keeps 1/rho in double beside them: one division a particle
-// instead of one a pair.
+// 2868; four steps of 4.2M in FP32 5020 for 4740); 1/rho uses force's recip.
+// FP64 keeps 1/rho in double beside them: one division a particle instead of
+// one a pair.
 __device__ __forceinline__ void load_pair(const PairRec* __restrict__ rec, float4& x, float4& v) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
@@ -630,7 +631,8 @@ __device__ __forceinline__ int scan_tile(
     const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const SceneDev* __restrict__ scenes,
     const float* __restrict__ wave, float2* __restrict__ rho_p, uint16_t* __restrict__ list,
     int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total,
-    int32_t* status, int32_t allow_stage, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho) {
+    int32_t* status, int32_t allow_stage, const float4* __restrict__ vel, PairRec* __restrict__ pairs,
+    double* __restrict__ irho) {
   using T = Real<P>;
   constexpr int kCap = kMaxVerlet;  // the Verlet list build's codes per particle
   // The list build (rare: Verlet rebuilds only) reads candidates from global
@@ -798,9 +800,9 @@ __global__ void __launch_bounds__(kNbThreads, MINB)
                  const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                  float2* __restrict__ rho_p, uint16_t* __restrict__ list, int32_t* __restrict__ list_cnt,
                  RowMask* __restrict__ masks, float4* __restrict__ xref, int32_t n_total, int32_t* status,
-                 const int32_t* __restrict__ flag,
-                 int32_t allow_stage, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho, const int32_t* __restrict__ order, int32_t* queue,
-                 int32_t n_tiles) {
+                 const int32_t* __restrict__ flag, int32_t allow_stage, const float4* __restrict__ vel,
+                 PairRec* __restrict__ pairs, double* __restrict__ irho, const int32_t* __restrict__ order,
+                 int32_t* queue, int32_t n_tiles) {
   __shared__ ScanShared<MODE> sh;
   __shared__ int32_t s_next;
   if (MODE == MODE_LIST && flag && __ldg(flag) == 0) return;  // no rebuild this step
@@ -836,7 +838,8 @@ __global__ void __launch_bounds__(kNbThreads, 8)
                const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                float2* __restrict__ rho_p, const uint16_t* __restrict__ vlist,
                const int32_t* __restrict__ vcnt, RowMask* __restrict__ nbm, int32_t* __restrict__ nbr_cnt,
-               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho) {
+               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs,
+               double* __restrict__ irho) {
   using T = Real<P>;
   __shared__ int32_t s_rb[9][kNbThreads];
   __shared__ RowMask s_m[kNbRows][kNbThreads];  // this step's row masks
@@ -1134,7 +1137,8 @@ __device__ __forceinline__ void force_tile(
     const float4* __restrict__ pos, const float2* __restrict__ rho_p,
     const int32_t* __restrict__ start, const int32_t* __restrict__ keys, const SceneDev* __restrict__ scenes,
     const float* __restrict__ wave, float4* __restrict__ force, const RowMask* __restrict__ nbm,
-    const int32_t* __restrict__ nbr_cnt, int32_t n_total, const PairRec* __restrict__ pairs, const double* __restrict__ irho, int32_t* status) {
+    const int32_t* __restrict__ nbr_cnt, int32_t n_total, const PairRec* __restrict__ pairs,
+    const double* __restrict__ irho, int32_t* status) {
   using T = Real<P>;
   const SceneDev* S = scenes + tl.scene;
   const int i = tl.begin + threadIdx.x;
@@ -1309,7 +1313,8 @@ __global__ void __launch_bounds__(kNbThreads)
     k_rho_team(const float4* __restrict__ pos, const int32_t* __restrict__ start, const int32_t* __restrict__ keys,
                const Tile* __restrict__ tiles, const SceneDev* __restrict__ scenes, const float* __restrict__ wave,
                float2* __restrict__ rho_p, int32_t* __restrict__ list_cnt, RowMask* __restrict__ masks,
-               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs, double* __restrict__ irho, int32_t* status) {
+               int32_t n_total, const float4* __restrict__ vel, PairRec* __restrict__ pairs,
+               double* __restrict__ irho, int32_t* status) {
   using R = Real<P>;
   const Tile tl = tiles[blockIdx.x / T];
   const int i = team_particle<T>(tl);
@@ -1545,7 +1550,8 @@ template <int P>
 void dispatch_scan(bool list_mode, const NbArgs& a, cudaStream_t st) {
   if (!list_mode && a.team) {
     k_rho_team<P, kTeamLanes><<<a.n_tiles * kTeamLanes, a.tile_size, 0, st>>>(
-        a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.pairs, a.irho, a.status);
+        a.pos, a.start, a.keys, a.tiles, a.scenes, a.wave, a.rho_p, a.nbr_cnt, a.nbm, a.n_total, a.vel, a.pairs,
+        a.irho, a.status);
     return;
   }
   if (list_mode)

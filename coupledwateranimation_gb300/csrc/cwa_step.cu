@@ -281,9 +281,12 @@ __global__ void k_wave_init(float* __restrict__ u, int32_t nx, int32_t nz, float
 constexpr int kLinkDepth = 8;
 constexpr int kLinkThreads = 256;
 constexpr int kLinkCtas = 32;
-// Up to 4 MB latency counts (a transfer takes ~20 us and the host waits for
-// it): one word a thread, and few registers, so that a CTA finds a place beside
-// other streams' kernels sooner.
+// Up to 4 MB latency counts (a transfer takes 15 to 34 us and the host waits
+// for it): one word a thread, and few registers, so that a CTA finds a place
+// beside other streams' kernels sooner: 64 scenes' uploads and eight steps took
+// 1% longer with the deep loads for these too.  Where the line lies between 64
+// KB and 4 MB made no difference to them, and alone an upload of any size takes
+// the same with either form (1 MB 19 us, 16 MB 93.5).
 constexpr long kLinkSmallWords = 1l << 18;
 
 // A warp reads 512 contiguous bytes (8 records' 16-byte quarters) of the source

@@ -271,7 +271,10 @@ cwa_status cwa_wave_init_from_image(cwa_sim* sim, int32_t scene, const uint8_t* 
  * (idle(), Main.cpp:549-560, plus the uniform-grid sort).  Asynchronous. */
 cwa_status cwa_step(cwa_sim* sim, int32_t n_steps);
 /* The same passes one at a time (one glDispatchCompute each).  cwa_pass_grid
- * must precede rho_pres in every step; the wave pass ends the step. */
+ * must precede rho_pres in every step; the wave pass ends the step.  Force
+ * takes its neighbours' state from records that rho_pres writes, in every
+ * precision: what a caller changes through a device view between the two is
+ * not seen by it. */
 cwa_status cwa_pass_grid(cwa_sim* sim);
 cwa_status cwa_pass_rho_pres(cwa_sim* sim);
 cwa_status cwa_pass_force(cwa_sim* sim);
@@ -391,7 +394,7 @@ cwa_status cwa_exclusive_scan_i32_noalloc(const int32_t* d_in, int32_t* d_out, i
 cwa_status cwa_scan_noalloc_status(void* stream);
 
 /* Uniform-grid build of n points (float4 xyz, stride 16 B): cell =
- * clamp(floor((p-lo)/cell), 0, dims-1), cell id (k*dims[1]+j)*dims[0]+i,
+ * clamp(floor((p-lo)/cell), 0, dims-1), cell id (i*dims[1]+j)*dims[2]+k,
  * stable counting sort.  Replaces the COMPUTE_COUNTS / scan / INSERT
  * sequence of UniformGridSph2D::CollisionQuery (SphWave2D/UniformGridGpu2D.cpp:220-265)
  * and UniformGrid2D/ugrid_particles_cs.glsl:90-117, with a deterministic
