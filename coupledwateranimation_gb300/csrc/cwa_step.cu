@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128)
                   cell_axis(pn.z, S->lo[2], S->cellz, nz);
     if (CWA_DCHECK_FAILED(k >= S->coff && k < S->coff + S->ncells, status)) return;
     key[i] = k;
-    slot[i] = count_slot(count, k);
+    slot[i] = count_slot_sorted(count, k);
   }
   if (xref) {  // Verlet mode: has this particle left its skin?
     const float4 r = xref[i];
