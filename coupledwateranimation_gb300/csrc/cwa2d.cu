@@ -907,6 +907,7 @@ cwa_status cwa2d_create(const cwa2d_params* p, int32_t device, cwa2d_sim** out) 
   const int nb = k.ncx * k.ncy + 1;  // grid cells + the bucket of points outside the grid
   auto fail = [&](cudaError_t e) {
     cwa::set_error(std::string("cwa2d_create: ") + cudaGetErrorString(e));
+    cudaGetLastError();  // clear a non-sticky error for the next call
     free2d(s);
     return e == cudaErrorMemoryAllocation ? CWA_ERR_OOM : CWA_ERR_CUDA;
   };

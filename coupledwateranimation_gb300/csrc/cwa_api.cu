@@ -167,6 +167,7 @@ cwa_status dev_alloc(cwa_sim* s, T** p, size_t count) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
   if (e != cudaSuccess) {
     set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    cudaGetLastError();  // clear a non-sticky error for the next call
     *p = nullptr;
     return CWA_ERR_OOM;
   }
@@ -923,6 +924,7 @@ cwa_status cwa_create(const cwa_sim_options* opt, const cwa_scene_desc* scenes, 
   s->ptile = o.nb_threads ? o.nb_threads : 128;
   s->verlet = o.verlet_skin > 0.0f;
   auto fail = [&](cwa_status st) {
+    cudaGetLastError();  // clear a non-sticky error for the next call
     free_sim(s);
     return st;
   };

@@ -643,6 +643,7 @@ cwa_status cwa_pbd_create(const cwa_pbd_params* p, int32_t device, cwa_pbd_sim**
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     cwa::set_error(std::string("cwa_pbd_create: ") + cudaGetErrorString(e));
+    cudaGetLastError();  // clear a non-sticky error for the next call
     free_pbd(s);
     return e == cudaErrorMemoryAllocation ? CWA_ERR_OOM : CWA_ERR_CUDA;
   }
