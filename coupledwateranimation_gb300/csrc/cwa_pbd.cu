@@ -534,10 +534,7 @@ cwa_status perr(const std::string& m, cwa_status s = CWA_ERR_INVALID_ARG) {
   } while (0)
 
 void free_items(cwa_pbd_sim* s) {
-  cudaFree(s->ikey);
-  cudaFree(s->islot);
-  cudaFree(s->clist);
-  cudaFree(s->csorted);
+  cudaFree(s->ikey);  // the four arrays are one allocation
   s->ikey = s->islot = s->clist = s->csorted = nullptr;
 }
 
@@ -680,12 +677,13 @@ cwa_status cwa_pbd_upload(cwa_pbd_sim* s, const cwa_pbd_box* host, int32_t n) {
       s->graph = nullptr;
     }
     free_items(s);
+    s->uploaded = false;  // no step until an upload has its buffers
     s->k.maxc = (int)maxc;
     const size_t items = (size_t)maxc * n;
-    PBD_CUDA(cudaMalloc((void**)&s->ikey, 4 * items));
-    PBD_CUDA(cudaMalloc((void**)&s->islot, 4 * items));
-    PBD_CUDA(cudaMalloc((void**)&s->clist, 4 * items));
-    PBD_CUDA(cudaMalloc((void**)&s->csorted, 4 * items));
+    PBD_CUDA(cudaMalloc((void**)&s->ikey, 16 * items));
+    s->islot = s->ikey + items;
+    s->clist = s->islot + items;
+    s->csorted = s->clist + items;
   }
   PBD_CUDA(cudaMemcpyAsync(s->boxes, host, sizeof(cwa_pbd_box) * n, cudaMemcpyHostToDevice, s->stream));
   PBD_CUDA(cudaStreamSynchronize(s->stream));
